@@ -501,6 +501,7 @@ struct astg_handle {
         launch_factor(d, J, P.omega, P.min_diag, epoch, st, &prof);
         bool owner = mixed || (J.pcActive && J.pcAsync);
         if (J.clusterSize > 0 || J.pcActive || mixed) launch_level_schedule(d, J, owner, st);
+        mixed = mixed && J.pcActive32;
         ck(cudaEventRecord(evA, st), "event");
         lastOuter = 0;
         if (mixed) lastOuter = launch_pcg_mixed(d, J, tol, maxIter, 8, st, &prof);
@@ -883,8 +884,7 @@ struct astg_handle {
     // driven by one host thread each.
     struct Lane {
         double *b = nullptr, *x = nullptr, *r = nullptr, *s = nullptr, *z = nullptr, *part = nullptr, *sc = nullptr;
-        double *rl = nullptr, *yl = nullptr;
-        float *rl32 = nullptr, *yl32 = nullptr, *e32 = nullptr, *r32 = nullptr, *s32 = nullptr, *z32 = nullptr,
+        float *e32 = nullptr, *r32 = nullptr, *s32 = nullptr, *z32 = nullptr,
               *q32 = nullptr;
         int *isc = nullptr, *done = nullptr, *hostDone = nullptr;
         unsigned long long* amax = nullptr;
@@ -903,10 +903,8 @@ struct astg_handle {
             L.isc = dalloc<int>(ISC_COUNT);
             L.amax = dalloc<unsigned long long>(1);
             L.done = dalloc<int>(1);
-            if (J.rl) L.rl = dalloc<double>(rows);
-            if (J.yl) L.yl = dalloc<double>(rows);
-            if (J.rl32) {
-                L.rl32 = dalloc<float>(rows); L.yl32 = dalloc<float>(rows); L.e32 = dalloc<float>(rows);
+            if (J.e32) {
+                L.e32 = dalloc<float>(rows);
                 L.r32 = dalloc<float>(rows); L.s32 = dalloc<float>(rows); L.z32 = dalloc<float>(rows);
                 L.q32 = dalloc<float>(rows);
             }
@@ -935,8 +933,7 @@ struct astg_handle {
         Proj Q = J;
         Q.b = L.b; Q.x = L.x; Q.r = L.r; Q.s = L.s; Q.z = L.z; Q.part = L.part; Q.sc = L.sc; Q.isc = L.isc;
         Q.amax = L.amax; Q.done = L.done; Q.hostDone = L.hostDone;
-        Q.rl = L.rl; Q.yl = L.yl;
-        Q.rl32 = L.rl32; Q.yl32 = L.yl32; Q.e32 = L.e32; Q.r32 = L.r32; Q.s32 = L.s32; Q.z32 = L.z32; Q.q32 = L.q32;
+        Q.e32 = L.e32; Q.r32 = L.r32; Q.s32 = L.s32; Q.z32 = L.z32; Q.q32 = L.q32;
         return Q;
     }
     void solveBatch(int n, const int32_t* rowptr, const int32_t* col, const double* val, int nrhs, const double* B,
@@ -960,10 +957,11 @@ struct astg_handle {
         select_preconditioner(J, n);
         launch_external_system(d, J, n, st);
         checkStatus();
-        const bool mixed = precision == ASTG_MIXED && J.pcActive32;
+        bool mixed = precision == ASTG_MIXED && J.pcActive32;
         launch_factor(d, J, P.omega, P.min_diag, epoch, st, nullptr);
         const bool owner = mixed || (J.pcActive && J.pcAsync);
         if (J.clusterSize > 0 || J.pcActive || mixed) launch_level_schedule(d, J, owner, st);
+        mixed = mixed && J.pcActive32;
         ck(cudaStreamSynchronize(st), "factor");
         checkStatus();
         // lanes only with the barrier-free preconditioner: the other forms hand rows out from one

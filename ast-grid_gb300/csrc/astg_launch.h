@@ -107,39 +107,46 @@ struct Proj {
     int pcCluster;   // CTAs per cluster of the fused DSMEM preconditioner (0: not available)
     int pcActive;    // the current solve uses it (its vector fits in the cluster's shared memory)
     size_t pcSmemMax;  // largest dynamic shared memory per CTA it may use
-    // padded level-ordered records for the fused preconditioner (entry e of row p at e * rowsCap + p)
+    // padded level-ordered records of the level-barrier fused preconditioner (entry e of row p at
+    // e * rowsCap + p)
     int rowsCap;
     int* pos;        // rows: level position of each row (inverse of perm)
     int* lcntF;      // rows: lower entries of the row at level position p
     int* lcntB;
     double* linvd;   // rows: pivot reciprocal in level order
     double* rl;      // rows: right-hand side of the preconditioner in level order
-    // barrier-free form: row j is computed by, and stored in, CTA (j >> lgB) mod CS; each CTA walks
-    // its own rows sorted by level (positions [ownStart[c], ownStart[c + 1]))
-    int pcAsync;     // 1: barrier-free fused preconditioner, 0: one cluster barrier per level
-    int pcLgBlock;   // log2 of the rows per ownership block: row j belongs to CTA (j >> lgB) mod CS
-    int* chunk;      // device scalar: shared-memory slots per CTA
-    int* ownStart;   // CS + 1: first position of each CTA's rows
-    int* lself;      // rows: local (shared-memory) index of the row at each position
-    double* yl;      // rows: forward-sweep result at each position
-    int* ownCnt;     // pcCluster * (rows + 1): rows per (owner CTA, level)
-    int* ownPtr;
-    int* ownFill;
     int* fcolP;      // PC_MAXE * rowsCap
     double* fvalP;
     int* bcolP;
     double* bvalP;
-    // mixed precision: FP32 copies of the matrix and of the factor records, FP32 inner vectors
+    int pcAsync;     // 1: barrier-free fused preconditioner, 0: one cluster barrier per level
+    // barrier-free form (k_precond_async): rows dealt to pcCS CTAs in blocks of pcBlock, the rows of a
+    // (CTA, level) segment cut into items of 32; [0] forward, [1] backward
+    int pcCS;        // CTAs of the current solve's cluster
+    int pcWarps;     // warps per CTA
+    int pcBlock;     // rows per ownership block
+    int pcChunk;     // shared-memory slots per CTA (without the one that holds 0)
+    int itemCap;     // items, and quads after the first, that the arrays hold per sweep
+    int* itemTotal;  // device: items, forward and backward quads after the first
+    int* ownCnt;     // pcCluster * (rows + 1): rows per segment
+    int* ownPtr;     // first row of each segment in perm
+    int* ownFill;
+    int* itemPtr;    // first item of each segment
+    int* permD[2];   // rows of each segment by descending entry count
+    int2* itemRange[2];  // first row in permD, rows
+    int* itXq[2];    // first quad after the first, per item
+    int4* itRow[2];  // row records, 32 per item (FP64)
+    int4* itRow32[2];
+    int4* itCol[2];  // first quads, 32 per item
+    double* itVal[2];
+    float* itVal32[2];
+    int4* itXcol[2];  // quads after the first
+    double* itXval[2];
+    float* itXval32[2];
+    // mixed precision: FP32 copy of the matrix, FP32 inner vectors
     int pcActive32;   // the current solve can run the FP32 barrier-free preconditioner
     size_t pcSmem32;  // its dynamic shared memory per CTA
     float* val32;     // rowsCap * ROW_W
-    float* fvalP32;   // PC_MAXE * rowsCap
-    float* bvalP32;
-    float* linvd32;
-    float* rl32;
-    float* yl32;
-    float* fval32;    // compact entries
-    float* bval32;
     float* e32;       // inner correction
     float* r32;       // inner residual
     float* s32;
@@ -250,7 +257,8 @@ void launch_velocity_ghost(const Dev& d, const Fields& F, const uint8_t* lastWri
 void launch_dof_numbering(const Dev& d, const uint8_t* open, Proj& P, cudaStream_t st);
 void launch_assemble(const Dev& d, const Fields& F, const uint8_t* open, Proj& P, const int* hoPtr, const int* hoIdx,
                      double dt, cudaStream_t st);
-// owner: the owner-major walk of the barrier-free preconditioner, else the level order
+// owner: the items of the barrier-free preconditioner, else the level order (also when the items do
+// not fit: P.pcActive and P.pcActive32 are then cleared)
 void launch_level_schedule(const Dev& d, Proj& P, bool owner, cudaStream_t st);
 void launch_external_system(const Dev& d, Proj& P, int rows, cudaStream_t st);
 // padded rows (rowCnt, padCol, padVal, bRaw over maxRows rows, *nDof set) -> CSR with b = bRaw *

@@ -1235,231 +1235,313 @@ __global__ void __launch_bounds__(256, 1) k_precond_dsmem(Proj P, double* z, int
     cl.sync();
 }
 // ---- barrier-free fused preconditioner.  Same vector placement idea (z in the distributed
-// shared memory of one cluster), but no barrier per level: CTA c computes the rows it stores
-// (rows [c * chunk, (c + 1) * chunk)), each thread takes every blockDim-th of its CTA's rows in
-// level order, and a row waits only for the entries it reads.  An entry's readiness is its own
-// value: every slot starts as PCA_EMPTY, a signalling-NaN bit pattern that no floating-point
-// operation produces (arithmetic on NaN returns a quiet NaN), and a single aligned 8-byte store
-// makes the value visible, so no separate flag is needed.  Deadlock cannot occur: every thread
-// walks its rows in non-decreasing level order, rows read only rows of strictly lower levels
-// (forward) or higher levels (backward, walked in reverse), and all CTAs of a cluster are
-// resident together.  Every wait is bounded; on timeout the kernel records DS_WAIT_TIMEOUT, stops
-// waiting everywhere and finishes with invalid values.  Per row the updates are the reference's,
-// in the reference's order, each one fused multiply-subtract.
-constexpr int PCA_THREADS = 256;
+// shared memory of one cluster), but no barrier per level: CTA c computes the rows it stores, and a
+// row waits only for the entries it reads.  An entry's readiness is its own value: every slot starts
+// as EMPTY, a signalling-NaN bit pattern that no floating-point operation produces (arithmetic on NaN
+// returns a quiet NaN), and a single aligned store makes the value visible, so no separate flag is
+// needed.
+//
+// The rows of one CTA and level are sorted by their entry count and cut into items of 32 rows, one
+// per lane; item k of a CTA's walk belongs to its warp k mod W.  An item's records are stored for
+// the warp that reads them: one 16-byte row record per lane, then its entries four at a time (a
+// quad: four packed columns, four factor values), right-aligned, so that a row shorter than the
+// item's longest starts with entries of value 0 that read a slot holding 0 (fma(-0, 0, acc) = acc).
+// Every load is one coalesced 16-byte load per lane with no branch on the row's length, the next
+// item's records are fetched while this one waits, and the rows of an item are of one level, so
+// their lanes become ready together and the arithmetic runs once for the whole warp.
+//
+// Deadlock cannot occur: every warp walks its items in non-decreasing level order, rows read only
+// rows of strictly lower levels (forward) or higher levels (backward, walked in reverse), and all
+// CTAs of a cluster are resident together.  Every wait is bounded; on timeout the kernel records
+// DS_WAIT_TIMEOUT, stops waiting everywhere and finishes with invalid values.  Per row the updates
+// are the reference's, in the reference's order, each one fused multiply-subtract.
+//
+// What bounds it: latency per level, from the store of a value to the store of a value that
+// depends on it.  Measured on GB300 for the 256^3-equivalent system (306,797 rows, 187 levels) per
+// application against the earlier form (one generic row per lane, up to 16 polled entries,
+// 256 threads): FP64 464 -> 222 us, FP32 330 -> 170 us; 42,797 rows (92 levels) FP64 82 us; 1,542
+// rows (28 levels) FP64 27 us.  What the measurements showed:
+// * The instructions of a row's path count, not its bytes: a lone warp issues a dependent
+//   instruction every ~5 cycles, so the earlier polling pass of ~400 instructions cost more than
+//   the chain it waited for.
+// * A predicated-off FP64 instruction costs a full one (~17 cycles of the SM's only FP64 pipe, 67 of
+//   latency).  The first quad is therefore entered by a jump (chain4), never by predicates.
+// * A wait for a fetched register also waits for later fetches that share its scoreboard; the
+//   fetched quad is read (look) before the next fetches are issued.
+// * The records bypass L1: at 150 KB of shared memory per CTA little L1 is left, and allocating
+//   there cost 7 % (238 -> 222 us).
+// * A scattered read of another CTA's slots takes ~3 cycles per lane, and 225 cycles at least, so
+//   rows are dealt in large blocks (select_preconditioner): 14 % of the entries cross CTAs instead of
+//   34 % with blocks of 256 rows.
 constexpr long long PCA_SPIN_LIMIT = 1LL << 22;
+constexpr int PCA_MAX_WARPS = 16;
 // Value-type traits of the barrier-free preconditioner (FP64 drop-in form, FP32 inner solve of the
-// mixed-precision form).  EMPTY is a signalling-NaN bit pattern: no floating-point operation
-// produces it (arithmetic on a NaN returns a quiet NaN).
+// mixed-precision form).  Slots are read with weak loads kept in place by asm volatile: shared
+// memory is not cached, so each one reads the slot's current contents, and an aligned store is seen
+// whole or not at all.  The value itself is the signal, so nothing else needs ordering; the
+// cluster barrier at the end of each sweep orders everything for what follows.
 template <typename T> struct Pca;
 template <> struct Pca<double> {
     typedef unsigned long long Bits;
     static constexpr Bits EMPTY = 0x7FF4DEADBEEF0001ull;
-    // Polls are plain (weak) loads of shared-memory slots kept in place by asm volatile: shared
-    // memory is not cached, so each one reads the slot's current contents, and an aligned store is seen
-    // whole or not at all.  The value itself is the signal, so nothing else needs ordering; the
-    // cluster barrier at the end of each sweep orders everything for what follows.  (Loads with
-    // .relaxed.cluster semantics measured about 20x slower per polling pass with every warp of
-    // the cluster polling.)
-    static __device__ __forceinline__ Bits ld(const void* a) {
+    // the high word alone: with these bits the value is a signalling NaN whatever its low word
+    static __device__ __forceinline__ bool empty(Bits b) { return (unsigned)(b >> 32) == (unsigned)(EMPTY >> 32); }
+    static __device__ __forceinline__ Bits ld(uint32_t a) {
         Bits v;
-        asm volatile("ld.b64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
+        asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
         return v;
+    }
+    static __device__ __forceinline__ void ld_if(Bits& v, uint32_t a, bool on) {
+        asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.shared::cluster.b64 %0, [%1];}" : "+l"(v) : "r"(a), "r"((int)on) : "memory");
     }
     static __device__ __forceinline__ void st(uint32_t a, double v) {
         asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"((Bits)__double_as_longlong(v)) : "memory");
     }
     static __device__ __forceinline__ double val(Bits b) { return __longlong_as_double((long long)b); }
+    // acc -= v[e] z[e] (fused) for the last w of four entries, in order
+    static __device__ __forceinline__ double chain4(double acc, int w, const double* v, const Bits* z) {
+        asm volatile(
+            "{ts_%=: .branchtargets L0_%=, L1_%=, L2_%=, L3_%=, L4_%=;\n\t"
+            "brx.idx.uni %1, ts_%=;\n\t"
+            "L4_%=: fma.rn.f64 %0, %2, %6, %0;\n\t"
+            "L3_%=: fma.rn.f64 %0, %3, %7, %0;\n\t"
+            "L2_%=: fma.rn.f64 %0, %4, %8, %0;\n\t"
+            "L1_%=: fma.rn.f64 %0, %5, %9, %0;\n\t"
+            "L0_%=:}"
+            : "+d"(acc)
+            : "r"(w), "d"(-v[0]), "d"(-v[1]), "d"(-v[2]), "d"(-v[3]), "d"(val(z[0])), "d"(val(z[1])), "d"(val(z[2])), "d"(val(z[3])));
+        return acc;
+    }
 };
 template <> struct Pca<float> {
     typedef unsigned int Bits;
     static constexpr Bits EMPTY = 0x7FA5DEADu;
-    static __device__ __forceinline__ Bits ld(const void* a) {
+    static __device__ __forceinline__ bool empty(Bits b) { return b == EMPTY; }
+    static __device__ __forceinline__ Bits ld(uint32_t a) {
         Bits v;
-        asm volatile("ld.b32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+        asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
         return v;
+    }
+    static __device__ __forceinline__ void ld_if(Bits& v, uint32_t a, bool on) {
+        asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.shared::cluster.b32 %0, [%1];}" : "+r"(v) : "r"(a), "r"((int)on) : "memory");
     }
     static __device__ __forceinline__ void st(uint32_t a, float v) {
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(__float_as_uint(v)) : "memory");
     }
     static __device__ __forceinline__ float val(Bits b) { return __uint_as_float(b); }
-};
-// per-precision arrays of the preconditioner (the schedule and columns are shared)
-template <typename T> struct PcaData {
-    const T* fvalP;  // PC_MAXE x rowsCap, level-ordered factor values (forward / backward)
-    const T* bvalP;
-    const T* linvd;  // pivot reciprocals at each position
-    const T* rl;     // right-hand side at each position
-    T* yl;           // forward result at each position
-    const T* fval;   // compact entries (read beyond PC_MAXE)
-    const T* bval;
-};
-template <typename T> struct PcaRow {
-    int p, self, cnt;
-    T rhs, invd;
-    int col[PC_MAXE];
-    T val[PC_MAXE];
-};
-// record of position p (valid when q < cnt): independent loads only
-template <typename T>
-__device__ __forceinline__ void pca_load(const Proj& P, const PcaData<T>& D, int base, int q, int rows, bool fwd,
-                                         PcaRow<T>& w) {
-    w.cnt = -1;
-    if (q < 0 || q >= rows) return;
-    const int p = base + q;
-    const int cap = P.rowsCap;
-    const int* cc = fwd ? P.fcolP : P.bcolP;
-    const T* vv = fwd ? D.fvalP : D.bvalP;
-    w.p = p;
-    w.self = P.lself[p];
-    w.cnt = fwd ? P.lcntF[p] : P.lcntB[p];
-    w.invd = D.linvd[p];
-    w.rhs = fwd ? D.rl[p] : D.yl[p];
+    static __device__ __forceinline__ float chain4(float acc, int w, const float* v, const Bits* z) {
 #pragma unroll
-    for (int e = 0; e < PC_MAXE; ++e) {
-        w.col[e] = cc[(size_t)e * cap + p];
-        w.val[e] = vv[(size_t)e * cap + p];
+        for (int e = 0; e < 4; ++e)
+            if (w >= 4 - e) acc = fmaf(-v[e], val(z[e]), acc);
+        return acc;
     }
+};
+// 16-byte load of a record that is read once per application: not kept in L1
+__device__ __forceinline__ int4 ld_rec(const void* p) {
+    int4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
-// One row per lane; the warp polls until every lane's row is done.  A lane stores its row the
-// moment its last entry arrives, so no lane ever waits for a lane of its own warp while holding its
-// own result back.  The loop and its exit are warp-uniform.  Entry addresses are resolved once per
-// row into generic addresses: a slot of the CTA's own shared memory is read there directly, a slot
-// of another CTA through the cluster's distributed shared memory, with one load form for both
-// (measured 2-3 % faster than routing every entry through the cluster window); every pass
-// re-loads all entries still missing, so they resolve in parallel.  Bounded: after PCA_SPIN_LIMIT
-// polls (or once any wait of the launch has given up) the warp stops waiting and reports.
-constexpr int PCA_MAXE = 2 * PC_MAXE;  // entries a row resolves in registers (8 from the record)
-// The polling pass is integer-only: it re-loads the entries not yet known to hold values and
-// extends the prefix of present ones.  The arithmetic runs once per row, after every entry is
-// present, in the reference's order (FP64 issue is scarce on this part, and predicated-off FP64
-// instructions in a polling pass would still occupy the FP64 pipe on every pass).
-// generic address of packed entry (owner << 24 | local): the CTA's own slots resolve to its shared
-// memory, other CTAs' slots to the cluster's distributed shared memory
+// row record of an item's lane: pivot reciprocal, row, local slot | quads << 24 | (entries of the
+// first quad - 1) << 28 | any entry in another CTA << 31 (the last three are the item's)
+template <typename T> struct PcaRow;
+template <> struct alignas(16) PcaRow<double> {
+    double invd;
+    int j;
+    unsigned f;
+};
+template <> struct alignas(16) PcaRow<float> {
+    float invd;
+    int j;
+    unsigned f;
+    int pad;
+};
+static_assert(sizeof(PcaRow<double>) == 16 && sizeof(PcaRow<float>) == 16, "row records are one 16-byte load");
 template <typename T>
-__device__ __forceinline__ const T* pca_gptr(T* const* win, int packed) {
-    return win[packed >> 24] + (packed & 0xffffff);
+__device__ __forceinline__ PcaRow<T> pca_row(const PcaRow<T>* p) {
+    int4 v = ld_rec(p);
+    return *reinterpret_cast<PcaRow<T>*>(&v);
 }
-template <typename T, bool UNFUSED>
-__device__ __forceinline__ void pca_solve_row(const Proj& P, const PcaData<T>& D, const PcaRow<T>& w, bool fwd,
-                                              uint32_t own, T* const* win, int* status) {
+__device__ __forceinline__ void pca_vals(const double* p, double* v) {
+    int4 a = ld_rec(p), b = ld_rec(p + 2);
+    double2 x = *reinterpret_cast<double2*>(&a), y = *reinterpret_cast<double2*>(&b);
+    v[0] = x.x;
+    v[1] = x.y;
+    v[2] = y.x;
+    v[3] = y.y;
+}
+__device__ __forceinline__ void pca_vals(const float* p, float* v) {
+    int4 a = ld_rec(p);
+    float4 x = *reinterpret_cast<float4*>(&a);
+    v[0] = x.x;
+    v[1] = x.y;
+    v[2] = x.z;
+    v[3] = x.w;
+}
+// a quad as fetched, and its entries' addresses and values
+template <typename T> struct PcaQuad {
+    int4 c;
+    T v[4];
+};
+template <typename T> struct PcaVals {
+    uint32_t a[4];
+    typename Pca<T>::Bits z[4];
+};
+template <typename T>
+__device__ __forceinline__ void pca_fetch(PcaQuad<T>& q, const int4* cols, const T* vals, size_t at) {
+    q.c = ld_rec(cols + at);
+    pca_vals(vals + 4 * at, q.v);
+}
+// first look at a quad's entries.  A column is the entry's slot, | owner CTA << 24 | 1 << 31 when the
+// owner is another CTA; only items with such entries look the owners' windows up.
+template <typename T>
+__device__ __forceinline__ void pca_look(const PcaQuad<T>& q, PcaVals<T>& s, uint32_t own, uint32_t win, bool remote) {
+    const int c[4] = {q.c.x, q.c.y, q.c.z, q.c.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s.a[e] = own + (uint32_t)(c[e] & 0xffffff) * (uint32_t)sizeof(T);
+    if (remote) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (c[e] < 0) {
+                uint32_t b;
+                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(b) : "r"(win + (((uint32_t)c[e] >> 22) & 0x3cu)) : "memory");
+                s.a[e] = b + (uint32_t)(c[e] & 0xffffff) * (uint32_t)sizeof(T);
+            }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s.z[e] = Pca<T>::ld(s.a[e]);
+}
+// until every lane's four entries hold values (the loop and its exit are warp-uniform); a pass reads
+// again only what was missing
+template <typename T>
+__device__ __forceinline__ void pca_wait(PcaVals<T>& s, int* status) {
     typedef Pca<T> K;
-    typedef typename K::Bits Bits;
-    const uint32_t es = sizeof(T);
-    bool done = w.cnt < 0;
-    const T* a[PCA_MAXE];
-    T val[PCA_MAXE];
-#pragma unroll
-    for (int e = 0; e < PC_MAXE; ++e) {
-        a[e] = pca_gptr(win, w.col[e]);
-        val[e] = w.val[e];
-    }
-    // entries 8..15 of a longer row: loaded once, together, before any polling
-    const int* oc = fwd ? P.fcol : P.bcol;
-    const T* ov = fwd ? D.fval : D.bval;
-    const int q0 = (!done && w.cnt > PC_MAXE) ? (fwd ? P.fptr : P.bptr)[w.p] : 0;
-#pragma unroll
-    for (int e = PC_MAXE; e < PCA_MAXE; ++e) {
-        bool has = e < w.cnt;
-        a[e] = pca_gptr(win, has ? oc[q0 + e] : 0);
-        val[e] = has ? ov[q0 + e] : T(0);
-    }
-    const int lim = min(w.cnt, PCA_MAXE);
-    Bits v[PCA_MAXE];
-    int got = 0;        // leading entries known to hold values
-    bool part = false;  // the first lim entries are accumulated (rows longer than PCA_MAXE)
-    T acc = w.rhs;
     for (long long it = 0;; ++it) {
-        if (!done) {
-            if (!part) {
-                const int g0 = got;
-#pragma unroll
-                for (int e = 0; e < PCA_MAXE; ++e)
-                    if (e >= g0 && e < lim) v[e] = K::ld(a[e]);
-#pragma unroll
-                for (int e = 0; e < PCA_MAXE; ++e)
-                    if (e == got && e < lim && v[e] != K::EMPTY) got = e + 1;
-                if (got == lim) {
-#pragma unroll
-                    for (int e = 0; e < PCA_MAXE; ++e) {
-                        if (e >= lim) break;
-                        acc = sweep_update(UNFUSED, acc, val[e], K::val(v[e]));
-                    }
-                    part = true;
-                }
-            }
-            // rows longer than PCA_MAXE entries: the rest one at a time from the compact arrays
-            while (part && got < w.cnt) {
-                Bits x = K::ld(pca_gptr(win, oc[q0 + got]));
-                if (x == K::EMPTY) break;
-                acc = sweep_update(UNFUSED, acc, ov[q0 + got], K::val(x));
-                ++got;
-            }
-            if (part && got >= w.cnt) {
-                T y = acc * w.invd;
-                if (fwd) D.yl[w.p] = y;
-                K::st(own + (uint32_t)w.self * es, y);
-                done = true;
-            }
-        }
-        if (__all_sync(0xffffffffu, done)) break;
+        const bool e0 = K::empty(s.z[0]), e1 = K::empty(s.z[1]), e2 = K::empty(s.z[2]), e3 = K::empty(s.z[3]);
+        if (!__any_sync(0xffffffffu, e0 | e1 | e2 | e3)) break;
         if ((it & 255) == 255) {
-            bool over = it > PCA_SPIN_LIMIT;
+            const bool over = it > PCA_SPIN_LIMIT;
             if (over) atomicCAS(status, 0, DS_WAIT_TIMEOUT);
             if (__any_sync(0xffffffffu, over || *(volatile int*)status != 0)) break;
         }
+        K::ld_if(s.z[0], s.a[0], e0);
+        K::ld_if(s.z[1], s.a[1], e1);
+        K::ld_if(s.z[2], s.a[2], e2);
+        K::ld_if(s.z[3], s.a[3], e3);
     }
 }
+// the updates of a quad's last w entries (w uniform over the warp)
 template <typename T, bool UNFUSED>
-__global__ void __launch_bounds__(PCA_THREADS, 1) k_precond_async(Proj P, PcaData<T> D, T* z, int* status, int lgCS) {
-    grid_dep_wait();
+__device__ __forceinline__ T pca_chain(T acc, int w, const PcaQuad<T>& q, const PcaVals<T>& s) {
+    if (!UNFUSED) return Pca<T>::chain4(acc, w, q.v, s.z);
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (w >= 4 - e) acc = sweep_update(true, acc, q.v[e], Pca<T>::val(s.z[e]));
+    return acc;
+}
+// One sweep's items: row records and first quads at (item * 32 + lane), the quads after the first at
+// ((xq[item] + q - 1) * 32 + lane)
+template <typename T> struct PcaDir {
+    const PcaRow<T>* row;
+    const int4* col;
+    const T* val;
+    const int* xq;
+    const int4* xcol;
+    const T* xval;
+};
+template <typename T> struct PcaData {
+    PcaDir<T> d[2];  // forward, backward
+    const int* itemPtr;  // first item of each (CTA, level), CTA-major
+    const int* nLevels;
+    int chunk;           // slots per CTA (slot `chunk` holds 0)
+};
+template <typename T, bool UNFUSED>
+__global__ void __launch_bounds__(PCA_MAX_WARPS * 32, 1)
+k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const int* doneFlag, int* status) {
     typedef Pca<T> K;
-    if (*P.done) return;
     extern __shared__ __align__(16) unsigned char pca_smem[];
-    typename K::Bits* zraw = reinterpret_cast<typename K::Bits*>(pca_smem);
-    T* zsh = reinterpret_cast<T*>(pca_smem);
+    __shared__ uint32_t win[16];  // the CTAs' windows of the vector
     cg::cluster_group cl = cg::this_cluster();
-    const int rank = cl.block_rank();
-    const int n = *P.nDof, chunk = *P.chunk;
-    const int base = P.ownStart[rank];
-    const int rows = P.ownStart[rank + 1] - base;
-    const int lgB = P.pcLgBlock;
-    const uint32_t own = (uint32_t)__cvta_generic_to_shared(pca_smem);
-    __shared__ T* win[16];
-    if (threadIdx.x < cl.num_blocks()) win[threadIdx.x] = cl.map_shared_rank(zsh, (int)threadIdx.x);
-    if (threadIdx.x == rank) win[threadIdx.x] = zsh;
-    for (int l = threadIdx.x; l < chunk; l += blockDim.x) zraw[l] = K::EMPTY;
+    const int rank = cl.block_rank(), nb = cl.num_blocks();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
+    const uint32_t own = (uint32_t)__cvta_generic_to_shared(pca_smem), winA = (uint32_t)__cvta_generic_to_shared(win);
+    if (threadIdx.x < nb) {
+        uint32_t m;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(own), "r"(threadIdx.x));
+        win[threadIdx.x] = m;
+    }
+    typename K::Bits* zraw = reinterpret_cast<typename K::Bits*>(pca_smem);
+    for (int l = threadIdx.x; l <= D.chunk; l += blockDim.x) zraw[l] = l == D.chunk ? (typename K::Bits)0 : K::EMPTY;
+    grid_dep_wait();
+    if (*doneFlag) return;
     cl.sync();  // every CTA is running and every slot of the cluster is empty
+    const int nl = *D.nLevels;
+    const int first = D.itemPtr[rank * nl], items = D.itemPtr[(rank + 1) * nl] - first;
+#pragma unroll 1
     for (int dir = 0; dir < 2; ++dir) {
-        const bool fwd = dir == 0;
-        // list index k of this CTA's walk -> position offset (forward: ascending levels, backward:
-        // descending)
-        auto qof = [&](int k) { return fwd ? k : rows - 1 - k; };
-        // thread t takes entries t, t + blockDim, ...: the same number of rounds for every thread,
-        // so warps stay whole; the next record is loaded while the current row waits
-        const int T_ = (int)blockDim.x;
-        const int rounds = (rows + T_ - 1) / T_;
-        auto pick = [&](int k) {
-            int q = threadIdx.x + k * T_;
-            return q < rows ? qof(q) : -1;
-        };
-        PcaRow<T> W, X;
-        pca_load(P, D, base, pick(0), rows, fwd, W);
-        for (int k = 0; k < rounds; ++k) {
-            pca_load(P, D, base, pick(k + 1), rows, fwd, X);
-            pca_solve_row<T, UNFUSED>(P, D, W, fwd, own, win, status);
-            W = X;
+        const PcaDir<T>& S = D.d[dir];
+        // forward: the residual; backward: the forward sweep's result, written by this CTA
+        const T* rhs = dir == 0 ? r : z;
+        if (wid < items) {
+            size_t at = (size_t)(first + wid) * 32 + lane;
+            PcaRow<T> m = pca_row(S.row + at);
+            PcaQuad<T> q;
+            pca_fetch(q, S.col, S.val, at);
+            int xq = __ldg(S.xq + first + wid);
+#pragma unroll 1
+            for (int k = wid; k < items; k += W) {
+                const PcaRow<T> row = m;
+                const PcaQuad<T> q1 = q;
+                const size_t x = (size_t)xq * 32 + lane;
+                const unsigned f = __shfl_sync(0xffffffffu, row.f, 0) >> 24;
+                const int nq = f & 15, w0 = ((f >> 4) & 3) + 1;
+                const bool remote = (f & 128) != 0;
+                PcaVals<T> s1, s2, s3;
+                if (nq > 0) pca_look(q1, s1, own, winA, remote);
+                asm volatile("" ::: "memory");  // the fetches below stay behind the use of q1
+                T acc = rhs[row.j];
+                const int kn = k + W < items ? k + W : k;  // the last item fetches itself again
+                at = (size_t)(first + kn) * 32 + lane;
+                m = pca_row(S.row + at);
+                xq = __ldg(S.xq + first + kn);
+                PcaQuad<T> q2, q3;
+                if (nq > 1) pca_fetch(q2, S.xcol, S.xval, x);
+                if (nq > 2) pca_fetch(q3, S.xcol, S.xval, x + 32);
+                pca_fetch(q, S.col, S.val, at);
+                if (nq > 0) {
+                    pca_wait(s1, status);
+                    acc = pca_chain<T, UNFUSED>(acc, w0, q1, s1);
+                }
+                if (nq > 1) {
+                    pca_look(q2, s2, own, winA, remote);
+                    if (nq > 2) pca_look(q3, s3, own, winA, remote);
+                    pca_wait(s2, status);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc = sweep_update(UNFUSED, acc, q2.v[e], K::val(s2.z[e]));
+                    if (nq > 2) {
+                        pca_wait(s3, status);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc = sweep_update(UNFUSED, acc, q3.v[e], K::val(s3.z[e]));
+#pragma unroll 1
+                        for (int u = 2; u < nq - 1; ++u) {  // rows of more than 12 entries
+                            pca_fetch(q2, S.xcol, S.xval, x + 32 * (size_t)u);
+                            pca_look(q2, s2, own, winA, remote);
+                            pca_wait(s2, status);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc = sweep_update(UNFUSED, acc, q2.v[e], K::val(s2.z[e]));
+                        }
+                    }
+                }
+                const T y = acc * row.invd;
+                K::st(own + (row.f & 0xffffffu) * (uint32_t)sizeof(T), y);
+                z[row.j] = y;
+            }
         }
         cl.sync();  // sweep finished everywhere (global and shared writes ordered at cluster scope)
-        if (fwd) {
-            for (int l = threadIdx.x; l < chunk; l += blockDim.x) zraw[l] = K::EMPTY;
+        if (dir == 0) {
+            for (int l = threadIdx.x; l < D.chunk; l += blockDim.x) zraw[l] = K::EMPTY;
             cl.sync();
         }
-    }
-    // local slot l holds row ((l >> lgB) << lgCS | rank) << lgB | (l mod B)
-    for (int l = threadIdx.x; l < chunk; l += blockDim.x) {
-        int j = ((((l >> lgB) << lgCS) | rank) << lgB) | (l & ((1 << lgB) - 1));
-        if (j < n) z[j] = zsh[l];
     }
 }
 // how many clusters of the barrier-free preconditioner (FP64 or FP32 form) can be resident at
@@ -1467,12 +1549,12 @@ __global__ void __launch_bounds__(PCA_THREADS, 1) k_precond_async(Proj P, PcaDat
 int precond_concurrency(const Proj& P, bool fp32) {
     if (P.pcCluster <= 0) return 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(P.pcCluster);
-    cfg.blockDim = dim3(PCA_THREADS);
+    cfg.gridDim = dim3(P.pcCS);
+    cfg.blockDim = dim3(P.pcWarps * 32);
     cfg.dynamicSmemBytes = fp32 ? P.pcSmem32 : P.pcSmem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = P.pcCluster;
+    at[0].val.clusterDim.x = P.pcCS;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
@@ -1503,16 +1585,16 @@ static cudaError_t launch_precond_dsmem(const Proj& P, const double* r, double* 
     return cudaLaunchKernelEx(&cfg, k_precond_dsmem, P, z, log2_exact(P.pcCluster));
 }
 template <typename T>
-static cudaError_t launch_precond_async(const Dev& d, const Proj& P, const PcaData<T>& D, T* z, size_t smem,
+static cudaError_t launch_precond_async(const Dev& d, const Proj& P, const PcaData<T>& D, const T* r, T* z, size_t smem,
                                        cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(P.pcCluster);
-    cfg.blockDim = dim3(PCA_THREADS);
+    cfg.gridDim = dim3(P.pcCS);
+    cfg.blockDim = dim3(P.pcWarps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = P.pcCluster;
+    at[0].val.clusterDim.x = P.pcCS;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_pdl
@@ -1520,11 +1602,17 @@ static cudaError_t launch_precond_async(const Dev& d, const Proj& P, const PcaDa
     cfg.attrs = at;
     cfg.numAttrs = 2;
     count_launch();
-    if (P.unfused) return cudaLaunchKernelEx(&cfg, k_precond_async<T, true>, P, D, z, d.status, log2_exact(P.pcCluster));
-    return cudaLaunchKernelEx(&cfg, k_precond_async<T, false>, P, D, z, d.status, log2_exact(P.pcCluster));
+    if (P.unfused) return cudaLaunchKernelEx(&cfg, k_precond_async<T, true>, D, r, z, (const int*)P.done, d.status);
+    return cudaLaunchKernelEx(&cfg, k_precond_async<T, false>, D, r, z, (const int*)P.done, d.status);
 }
 static PcaData<double> pca_data64(const Proj& P) {
-    return PcaData<double>{P.fvalP, P.bvalP, P.linvd, P.rl, P.yl, P.fval, P.bval};
+    PcaData<double> D{};
+    for (int k = 0; k < 2; ++k)
+        D.d[k] = PcaDir<double>{(const PcaRow<double>*)P.itRow[k], P.itCol[k], P.itVal[k], P.itXq[k], P.itXcol[k], P.itXval[k]};
+    D.itemPtr = P.itemPtr;
+    D.nLevels = P.nLevels;
+    D.chunk = P.pcChunk;
+    return D;
 }
 // Cluster size (16, else 8) at which the fused preconditioner (barrier-free form when async) can
 // run with the largest dynamic shared memory a CTA may have, or 0; *smemMax = that largest size.
@@ -1532,7 +1620,7 @@ static PcaData<double> pca_data64(const Proj& P) {
 // when they do not fit.
 int choose_dsmem_cluster(bool async, size_t* smemMax) {
     const void* kern = async ? (const void*)k_precond_async<double, false> : (const void*)k_precond_dsmem;
-    const int threads = async ? PCA_THREADS : PC_THREADS;
+    const int threads = async ? PCA_MAX_WARPS * 32 : PC_THREADS;
     *smemMax = 0;
     cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     int dev = 0, optin = 0;
@@ -1630,115 +1718,198 @@ int choose_cluster_size(int device) {
     }
     return 0;
 }
-// ---- owner-major schedule of the barrier-free preconditioner.  Rows are dealt to the CTAs in
-// blocks of B = 2^lgB consecutive rows, round robin: row j is computed by, and keeps its value in,
-// CTA (j >> lgB) mod CS at local slot ((j >> (lgB + lgCS)) << lgB) | (j mod B).  Consecutive rows
-// (x neighbours, mostly y neighbours) share a CTA while every dependency level is spread over
-// all CTAs.  Each CTA's rows are sorted by level, so a row's dependencies always come earlier in
-// some CTA's walk.  Keys (owner, level) are counted, scanned and scattered.
-__device__ __forceinline__ int own_of(int j, int lgB, int lgCS) { return (j >> lgB) & ((1 << lgCS) - 1); }
-__device__ __forceinline__ int local_of(int j, int lgB, int lgCS) {
-    return ((j >> (lgB + lgCS)) << lgB) | (j & ((1 << lgB) - 1));
+// ---- item schedule of the barrier-free preconditioner (see k_precond_async), rebuilt per solve.
+// Rows are dealt to the CTAs in blocks of B rows, round robin: row j is computed by, and keeps its
+// value in, CTA (j / B) mod CS.  Segments (CTA, level) are counted, scanned and filled; each one's
+// rows are sorted by entry count, once per sweep, and cut into items of 32.
+__device__ __forceinline__ int own_of(const Proj& P, int j) { return (j / P.pcBlock) % P.pcCS; }
+__device__ __forceinline__ int slot_of(const Proj& P, int j) {
+    const int h = j / P.pcBlock;
+    return (h / P.pcCS) * P.pcBlock + (j - h * P.pcBlock);
 }
-// column k as (owner CTA << 24 | local slot)
-__device__ __forceinline__ int pack_owner(int k, int lgB, int lgCS) {
-    return (own_of(k, lgB, lgCS) << 24) | local_of(k, lgB, lgCS);
+__global__ void k_seg_levels(Proj P) {
+    int g = 0;
+    const int n = *P.nDof;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) g = max(g, P.level[j] + 1);
+    g = __reduce_max_sync(0xffffffffu, g);
+    if ((threadIdx.x & 31) == 0 && g > 0) atomicMax(P.nLevels, g);
 }
-__global__ void k_own_setup(Proj P, int cs, long long keys) {
-    long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < keys) { P.ownCnt[j] = 0; P.ownFill[j] = 0; }
-    if (j == 0) {
-        int B = 1 << P.pcLgBlock;
-        int blocks = (*P.nDof + B - 1) / B;
-        *P.chunk = ((blocks + cs - 1) / cs) * B;
+__global__ void k_seg_clear(Proj P) {
+    const long long keys = (long long)P.pcCS * *P.nLevels;
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < keys; k += (long long)gridDim.x * blockDim.x) {
+        P.ownCnt[k] = 0;
+        P.ownFill[k] = 0;
     }
+    if (blockIdx.x == 0 && threadIdx.x < 3) P.itemTotal[threadIdx.x] = 0;
 }
-__global__ void k_own_hist(Proj P, int rows1, int lgCS) {
+__global__ void k_seg_hist(Proj P) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= *P.nDof) return;
-    atomicAdd(P.ownCnt + (long long)own_of(j, P.pcLgBlock, lgCS) * rows1 + P.level[j], 1);
+    atomicAdd(P.ownCnt + (long long)own_of(P, j) * *P.nLevels + P.level[j], 1);
 }
-__global__ void k_own_scatter(Proj P, int rows1, int lgCS) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= *P.nDof) return;
-    long long key = (long long)own_of(j, P.pcLgBlock, lgCS) * rows1 + P.level[j];
-    int p = P.ownPtr[key] + atomicAdd(P.ownFill + key, 1);
-    P.perm[p] = j;
-    P.pos[j] = p;
-}
-__global__ void k_own_bounds(Proj P, int rows1, int cs) {
-    int c = threadIdx.x;
-    if (c < cs) P.ownStart[c] = P.ownPtr[(long long)c * rows1];
-    if (c == cs) P.ownStart[cs] = *P.nDof;
-}
-__global__ void k_own_fill(Proj P, int lgCS) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= *P.nDof) return;
-    int i = P.perm[p];
-    int dg = P.diagPos[i];
-    int lgB = P.pcLgBlock;
-    int cap = P.rowsCap;
-    P.lself[p] = local_of(i, lgB, lgCS);
-    P.linvd[p] = P.invdiag[i];
-    int nf = dg - P.rowPtr[i], nb = P.rowPtr[i + 1] - dg - 1;
-    P.lcntF[p] = nf;
-    P.lcntB[p] = nb;
-    P.cntF[p] = nf;
-    P.cntB[p] = nb;
-    for (int e = 0; e < PC_MAXE; ++e) {
-        int qf = P.rowPtr[i] + e, qb = dg + 1 + e;
-        P.fcolP[(size_t)e * cap + p] = e < nf ? pack_owner(P.col[qf], lgB, lgCS) : 0;
-        P.fvalP[(size_t)e * cap + p] = e < nf ? P.Lv[P.tpos[qf]] : 0.0;
-        P.bcolP[(size_t)e * cap + p] = e < nb ? pack_owner(P.col[qb], lgB, lgCS) : 0;
-        P.bvalP[(size_t)e * cap + p] = e < nb ? P.Lv[qb] : 0.0;
-        if (P.fvalP32) {  // the factor is computed in FP64 and rounded once
-            P.fvalP32[(size_t)e * cap + p] = (float)P.fvalP[(size_t)e * cap + p];
-            P.bvalP32[(size_t)e * cap + p] = (float)P.bvalP[(size_t)e * cap + p];
+// exclusive scans over the segments of their rows and of their items (one block: a few thousand
+// segments)
+__global__ void k_seg_scan(Proj P) {
+    __shared__ int sr[1024], si[1024];
+    const int t = threadIdx.x;
+    const long long keys = (long long)P.pcCS * *P.nLevels;
+    int br = 0, bi = 0;
+    for (long long k0 = 0; k0 < keys; k0 += 1024) {
+        const long long k = k0 + t;
+        const int c = k < keys ? P.ownCnt[k] : 0, m = (c + 31) >> 5;
+        sr[t] = c;
+        si[t] = m;
+        __syncthreads();
+        for (int s = 1; s < 1024; s <<= 1) {
+            const int a = t >= s ? sr[t - s] : 0, b = t >= s ? si[t - s] : 0;
+            __syncthreads();
+            sr[t] += a;
+            si[t] += b;
+            __syncthreads();
         }
+        if (k < keys) {
+            P.ownPtr[k] = br + sr[t] - c;
+            P.itemPtr[k] = bi + si[t] - m;
+        }
+        br += sr[1023];
+        bi += si[1023];
+        __syncthreads();
     }
-    if (P.linvd32) P.linvd32[p] = (float)P.invdiag[i];
-}
-// all entries of the row at position p, packed, in the compact arrays (read beyond PC_MAXE)
-__global__ void k_own_overflow(Proj P, int lgCS) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= *P.nDof) return;
-    int i = P.perm[p];
-    int dg = P.diagPos[i];
-    int lgB = P.pcLgBlock;
-    int o = P.fptr[p];
-    for (int q = P.rowPtr[i]; q < dg; ++q, ++o) {
-        P.fcol[o] = pack_owner(P.col[q], lgB, lgCS);
-        P.fval[o] = P.Lv[P.tpos[q]];
-        if (P.fval32) P.fval32[o] = (float)P.fval[o];
-    }
-    o = P.bptr[p];
-    for (int q = dg + 1; q < P.rowPtr[i + 1]; ++q, ++o) {
-        P.bcol[o] = pack_owner(P.col[q], lgB, lgCS);
-        P.bval[o] = P.Lv[q];
-        if (P.bval32) P.bval32[o] = (float)P.bval[o];
+    if (t == 0) {
+        P.ownPtr[keys] = br;
+        P.itemPtr[keys] = bi;
+        P.itemTotal[0] = bi;
     }
 }
-static void launch_owner_schedule(const Dev& d, Proj& P, cudaStream_t st) {
-    (void)d;
-    int maxRows = P.rowsCap;
-    int cs = P.pcCluster, lgCS = log2_exact(cs);
-    long long keys = (long long)cs * (maxRows + 1);
-    ASTG_LAUNCH(k_own_setup<<<nblk(keys), TB, 0, st>>>(P, cs, keys));
-    ASTG_LAUNCH(k_own_hist<<<nblk(maxRows), TB, 0, st>>>(P, maxRows + 1, lgCS));
-    exclusive_scan(P.ownCnt, P.ownPtr, P.bsum, P.nnz + 1, keys, st);
-    ASTG_LAUNCH(k_own_bounds<<<1, 32, 0, st>>>(P, maxRows + 1, cs));
-    ASTG_LAUNCH(k_own_scatter<<<nblk(maxRows), TB, 0, st>>>(P, maxRows + 1, lgCS));
-    ASTG_LAUNCH(k_own_fill<<<nblk(maxRows), TB, 0, st>>>(P, lgCS));
-    exclusive_scan(P.cntF, P.fptr, P.bsum, P.nnz + 2, maxRows, st);
-    exclusive_scan(P.cntB, P.bptr, P.bsum, P.nnz + 3, maxRows, st);
-    ASTG_LAUNCH(k_level_fptr_last<<<1, 1, 0, st>>>(P));
-    ASTG_LAUNCH(k_own_overflow<<<nblk(maxRows), TB, 0, st>>>(P, lgCS));
+__global__ void k_seg_scatter(Proj P) {
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= *P.nDof) return;
+    const long long key = (long long)own_of(P, j) * *P.nLevels + P.level[j];
+    P.perm[P.ownPtr[key] + atomicAdd(P.ownFill + key, 1)] = j;
+}
+// one warp per segment: its rows by descending entry count (a counting sort), and its items' ranges.
+// The backward sweep walks a CTA's levels in reverse, so its items are numbered from the CTA's end.
+__global__ void k_seg_sort(Proj P, int dir) {
+    __shared__ int bins[8][ROW_W];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nl = *P.nLevels;
+    const long long keys = (long long)P.pcCS * nl;
+    if (P.itemTotal[0] > P.itemCap) return;
+    for (long long k = (long long)blockIdx.x * 8 + w; k < keys; k += (long long)gridDim.x * 8) {
+        const int p0 = P.ownPtr[k], m = P.ownPtr[k + 1] - p0;
+        if (m == 0) continue;
+        bins[w][lane] = 0;
+        __syncwarp();
+        auto count = [&](int i) {
+            const int dg = P.diagPos[i];
+            return dir == 0 ? dg - P.rowPtr[i] : P.rowPtr[i + 1] - dg - 1;
+        };
+        for (int e = lane; e < m; e += 32) atomicAdd(&bins[w][ROW_W - 1 - count(P.perm[p0 + e])], 1);
+        __syncwarp();
+        const int c = bins[w][lane];
+        int incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        bins[w][lane] = incl - c;
+        __syncwarp();
+        for (int e = lane; e < m; e += 32) {
+            const int i = P.perm[p0 + e];
+            P.permD[dir][p0 + atomicAdd(&bins[w][ROW_W - 1 - count(i)], 1)] = i;
+        }
+        const int n = (m + 31) >> 5;
+        const int cta = (int)(k / nl);
+        const int id0 = dir == 0 ? P.itemPtr[k] : P.itemPtr[(long long)cta * nl] + P.itemPtr[(long long)(cta + 1) * nl] - P.itemPtr[k] - n;
+        for (int u = lane; u < n; u += 32) P.itemRange[dir][id0 + u] = make_int2(p0 + 32 * u, min(32, m - 32 * u));
+        __syncwarp();
+    }
+}
+// one warp per item: the records of its 32 lanes (lanes past its last row repeat that row)
+__global__ void k_item_fill(Proj P, int dir) {
+    const int item = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const int total = P.itemTotal[0];
+    if (total > P.itemCap || item >= total) return;
+    const int2 rg = P.itemRange[dir][item];
+    const int i = P.permD[dir][rg.x + min(lane, rg.y - 1)];
+    const int dg = P.diagPos[i];
+    const int q0 = dir == 0 ? P.rowPtr[i] : dg + 1, q1 = dir == 0 ? dg : P.rowPtr[i + 1];
+    const int cnt = q1 - q0;
+    const int longest = __reduce_max_sync(0xffffffffu, cnt);
+    const int nq = (longest + 3) >> 2, w0 = nq ? longest - 4 * (nq - 1) : 1;
+    int x = 0;
+    if (nq > 1) {
+        if (lane == 0) x = atomicAdd(P.itemTotal + 1 + dir, nq - 1);
+        x = __shfl_sync(0xffffffffu, x, 0);
+        if (x + nq - 1 > P.itemCap) return;  // the host reads the totals and takes another form
+    }
+    if (lane == 0) P.itXq[dir][item] = x;
+    const int self = own_of(P, i);
+    bool remote = false;
+    for (int u = 0; u < max(nq, 1); ++u) {
+        int c[4];
+        double v[4];
+        for (int e = 0; e < 4; ++e) {
+            const int q = q0 + 4 * u + e - (4 * nq - cnt);  // right-aligned
+            c[e] = P.pcChunk;
+            v[e] = 0;
+            if (u < nq && q >= q0 && q < q1) {
+                const int k = P.col[q], o = own_of(P, k);
+                c[e] = slot_of(P, k);
+                if (o != self) {
+                    c[e] |= (o << 24) | (int)0x80000000u;
+                    remote = true;
+                }
+                v[e] = dir == 0 ? P.Lv[P.tpos[q]] : P.Lv[q];
+            }
+        }
+        const size_t at = (size_t)(u == 0 ? item : x + u - 1) * 32 + lane;
+        (u == 0 ? P.itCol : P.itXcol)[dir][at] = make_int4(c[0], c[1], c[2], c[3]);
+        double2* dv = reinterpret_cast<double2*>((u == 0 ? P.itVal : P.itXval)[dir] + 4 * at);
+        dv[0] = make_double2(v[0], v[1]);
+        dv[1] = make_double2(v[2], v[3]);
+        // the factor is computed in FP64 and rounded once
+        *reinterpret_cast<float4*>((u == 0 ? P.itVal32 : P.itXval32)[dir] + 4 * at) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+    }
+    const unsigned f = (unsigned)slot_of(P, i) | ((unsigned)(nq | ((w0 - 1) << 4) | (__any_sync(0xffffffffu, remote) ? 128 : 0)) << 24);
+    const size_t at = (size_t)item * 32 + lane;
+    PcaRow<double> r;
+    r.invd = P.invdiag[i];
+    r.j = i;
+    r.f = f;
+    ((PcaRow<double>*)P.itRow[dir])[at] = r;
+    PcaRow<float> r32;
+    r32.invd = (float)P.invdiag[i];
+    r32.j = i;
+    r32.f = f;
+    r32.pad = 0;
+    ((PcaRow<float>*)P.itRow32[dir])[at] = r32;
+}
+// false when the items do not fit their arrays (a matrix of very many, very narrow levels): the
+// caller takes another form of the sweeps
+static bool launch_item_schedule(Proj& P, cudaStream_t st) {
+    const int maxRows = P.rowsCap;
+    cudaMemsetAsync(P.nLevels, 0, sizeof(int), st);
+    ASTG_LAUNCH(k_seg_levels<<<std::min(nblk(maxRows), 512), TB, 0, st>>>(P));
+    ASTG_LAUNCH(k_seg_clear<<<64, TB, 0, st>>>(P));
+    ASTG_LAUNCH(k_seg_hist<<<nblk(maxRows), TB, 0, st>>>(P));
+    ASTG_LAUNCH(k_seg_scan<<<1, 1024, 0, st>>>(P));
+    ASTG_LAUNCH(k_seg_scatter<<<nblk(maxRows), TB, 0, st>>>(P));
+    for (int dir = 0; dir < 2; ++dir) {
+        ASTG_LAUNCH(k_seg_sort<<<512, TB, 0, st>>>(P, dir));
+        ASTG_LAUNCH(k_item_fill<<<nblk((long long)P.itemCap * 32), TB, 0, st>>>(P, dir));
+    }
+    int total[3] = {0, 0, 0};
+    cudaMemcpyAsync(total, P.itemTotal, sizeof total, cudaMemcpyDeviceToHost, st);
+    cudaStreamSynchronize(st);
+    return total[0] <= P.itemCap && total[1] <= P.itemCap && total[2] <= P.itemCap;
 }
 
 void launch_level_schedule(const Dev& d, Proj& P, bool owner, cudaStream_t st) {
     if (owner) {
-        launch_owner_schedule(d, P, st);
-        return;
+        if (launch_item_schedule(P, st)) return;
+        P.pcActive = 0;  // the level-synchronous sweeps, in level order
+        P.pcActive32 = 0;
+        if (P.clusterSize <= 0) return;
     }
     int maxRows = P.rowsCap;
     ASTG_LAUNCH(k_level_reset<<<nblk(maxRows + 1), TB, 0, st>>>(P, maxRows));
@@ -1940,7 +2111,7 @@ __global__ void k_update_xr(Proj P, double* x, double* r, const double* s, const
         x[i] = mac_add<FUSED>(x[i], alpha, s[i]);
         double ri = mac_add<FUSED>(r[i], -alpha, z[i]);
         r[i] = ri;
-        if (P.pcActive) P.rl[P.pos[i]] = ri;
+        if (P.rl && P.pcActive) P.rl[P.pos[i]] = ri;  // level-barrier form
         if (P.wave) wave_put_r(P, i, ri);
         v = fabs(ri);
     }
@@ -1993,21 +2164,28 @@ void select_preconditioner(Proj& P, int n) {
     P.pcSmem = 0;
     P.pcActive32 = 0;
     P.pcSmem32 = 0;
-    if (P.pcCluster <= 0 || n <= 0) return;
-    size_t slots = (size_t)((n + P.pcCluster - 1) / P.pcCluster);
-    if (P.pcAsync) {  // whole ownership blocks per CTA
-        size_t B = (size_t)1 << P.pcLgBlock, blocks = (n + B - 1) / B;
-        slots = (blocks + P.pcCluster - 1) / P.pcCluster * B;
+    if (P.pcCluster <= 0 || n <= 0 || n > P.rowsCap) return;
+    if (!P.pcAsync) {
+        size_t bytes = (size_t)((n + P.pcCluster - 1) / P.pcCluster) * sizeof(double);
+        if (bytes > P.pcSmemMax) return;
+        P.pcActive = 1;
+        P.pcSmem = bytes;
+        return;
     }
-    size_t bytes = slots * sizeof(double);
-    if (n > P.rowsCap) return;
-    if (P.pcAsync && P.val32 && slots * sizeof(float) <= P.pcSmemMax) {
+    const bool large = n > 100000;
+    P.pcWarps = large ? 12 : 8;
+    P.pcCS = n > 4096 ? P.pcCluster : 1;
+    const int blocks = large ? 3 : 1;
+    P.pcBlock = (n + P.pcCS * blocks - 1) / (P.pcCS * blocks);
+    P.pcChunk = P.pcBlock * blocks;
+    const size_t slots = (size_t)P.pcChunk + 1;  // and the slot that holds 0
+    if (slots * sizeof(float) <= P.pcSmemMax) {
         P.pcActive32 = 1;
         P.pcSmem32 = slots * sizeof(float);
     }
-    if (bytes > P.pcSmemMax) return;
+    if (slots * sizeof(double) > P.pcSmemMax) return;
     P.pcActive = 1;
-    P.pcSmem = bytes;
+    P.pcSmem = slots * sizeof(double);
 }
 static void precond(const Dev& d, Proj& P, const double* r, double* z, int& epoch, cudaStream_t st, KProf* prof) {
     if (P.wave) {
@@ -2018,7 +2196,7 @@ static void precond(const Dev& d, Proj& P, const double* r, double* z, int& epoc
     }
     if (P.pcActive) {
         prof_begin(prof, 0, st);
-        cudaError_t e = P.pcAsync ? launch_precond_async(d, P, pca_data64(P), z, P.pcSmem, st)
+        cudaError_t e = P.pcAsync ? launch_precond_async(d, P, pca_data64(P), r, z, P.pcSmem, st)
                                   : launch_precond_dsmem(P, r, z, st);
         prof_end(prof, st);
         if (e != cudaSuccess) g_cluster_error = e;
@@ -2213,7 +2391,7 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
     cudaMemsetAsync(P.amax, 0, sizeof(unsigned long long), st);
     cudaMemsetAsync(P.done, 0, sizeof(int), st);
     ASTG_LAUNCH(k_absmax<<<nblk(maxRows), TB, 0, st>>>(r, P.nDof, P.amax));
-    if (P.pcActive) ASTG_LAUNCH(k_to_level_order<<<nblk(maxRows), TB, 0, st>>>(P, r));
+    if (P.rl && P.pcActive) ASTG_LAUNCH(k_to_level_order<<<nblk(maxRows), TB, 0, st>>>(P, r));
     if (P.wave) ASTG_LAUNCH(k_to_wave_order<<<nblk(maxRows), TB, 0, st>>>(P, r));
     precond(d, P, r, z, epoch, st, prof);
     if (P.refOrder) launch_dot_ref(z, r, P.nDof, P.part, st);
@@ -2288,13 +2466,12 @@ __global__ void k_resid64(Proj P, const double* x, double* r) {
     }
     block_absmax_to(v, P.amax);
 }
-// start of an inner solve: r32 = r (also in walk order), e32 = 0
+// start of an inner solve: r32 = r, e32 = 0
 __global__ void k_inner_init(Proj P, const double* r) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *P.nDof) return;
     float ri = (float)r[i];
     P.r32[i] = ri;
-    P.rl32[P.pos[i]] = ri;
     P.e32[i] = 0.0f;
 }
 // partial dots of FP32 vectors, products and sums in FP64 (fixed tree)
@@ -2365,7 +2542,6 @@ __global__ void k_update_er32(Proj P) {
         P.e32[i] = fmaf(alpha, P.s32[i], P.e32[i]);
         float ri = fmaf(-alpha, P.q32[i], P.r32[i]);
         P.r32[i] = ri;
-        P.rl32[P.pos[i]] = ri;
         v = fabs((double)ri);
     }
     block_absmax_to(v, P.amax);
@@ -2386,7 +2562,13 @@ __global__ void k_mixed_finish(Proj P, double res, double tolAbs, double res0, i
     P.isc[ISC_CONVERGED] = converged;
 }
 static PcaData<float> pca_data32(const Proj& P) {
-    return PcaData<float>{P.fvalP32, P.bvalP32, P.linvd32, P.rl32, P.yl32, P.fval32, P.bval32};
+    PcaData<float> D{};
+    for (int k = 0; k < 2; ++k)
+        D.d[k] = PcaDir<float>{(const PcaRow<float>*)P.itRow32[k], P.itCol[k], P.itVal32[k], P.itXq[k], P.itXcol[k], P.itXval32[k]};
+    D.itemPtr = P.itemPtr;
+    D.nLevels = P.nLevels;
+    D.chunk = P.pcChunk;
+    return D;
 }
 static double read_amax(Proj& P, cudaStream_t st) {
     unsigned long long bits = 0;
@@ -2427,7 +2609,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
         ASTG_LAUNCH(k_inner_init<<<nblk(maxRows), TB, 0, st>>>(P, r));
         cudaMemsetAsync(P.done, 0, sizeof(int), st);
         prof_begin(prof, 0, st);
-        cudaError_t e = launch_precond_async(d, P, D, P.z32, P.pcSmem32, st);
+        cudaError_t e = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
         prof_end(prof, st);
         if (e != cudaSuccess) g_cluster_error = e;
         ASTG_LAUNCH(k_tree_dot32<<<chunks, RED_LANES, 0, st>>>(P.z32, P.r32, P.nDof, P.part));
@@ -2442,7 +2624,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
                 ASTG_LAUNCH(k_update_er32<<<nblk(maxRows), TB, 0, st>>>(P));
                 ASTG_LAUNCH(k_check<<<1, 1, 0, st>>>(P, maxIter));
                 prof_begin(pf, 0, st);
-                cudaError_t pe = launch_precond_async(d, P, D, P.z32, P.pcSmem32, st);
+                cudaError_t pe = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
                 prof_end(pf, st);
                 if (pe != cudaSuccess) g_cluster_error = pe;
                 ASTG_LAUNCH(k_tree_dot32<<<chunks, RED_LANES, 0, st>>>(P.z32, P.r32, P.nDof, P.part));
@@ -2542,33 +2724,39 @@ void proj_alloc(Proj& J, long long rows, int device, cudaStream_t st, std::vecto
     J.pcCluster = (mode == "async" || mode == "dsmem") ? choose_dsmem_cluster(J.pcAsync, &J.pcSmemMax) : 0;
     J.pcActive = 0;
     J.pcSmem = 0;
-    J.pcLgBlock = 8;  // 256-row ownership blocks (measured: 64 to 4096 within 3 %)
-    long long scanMax = std::max(rows * ROW_W + 1, (long long)std::max(J.pcCluster, 1) * (rows + 1));
-    J.bsum = A.get<int>((scanMax + 1023) / 1024 + 1);
+    J.bsum = A.get<int>((rows * ROW_W + 1 + 1023) / 1024 + 1);
     if (J.pcCluster && J.pcAsync) {
-        J.chunk = A.get<int>(1);
-        J.ownStart = A.get<int>(J.pcCluster + 1);
+        // items: 32 rows each where levels are wide, at least one per level and CTA; a sixteenth of the
+        // rows is twice what the octree systems take (all of them on small handles)
+        J.itemCap = (int)std::max(std::min(rows, 32768LL), rows / 16);
+        const long long L = 32LL * J.itemCap;
+        for (int k = 0; k < 2; ++k) {
+            J.permD[k] = A.get<int>(rows);
+            J.itemRange[k] = A.get<int2>(J.itemCap);
+            J.itXq[k] = A.get<int>(J.itemCap);
+            J.itRow[k] = A.get<int4>(L);
+            J.itRow32[k] = A.get<int4>(L);
+            J.itCol[k] = A.get<int4>(L);
+            J.itXcol[k] = A.get<int4>(L);
+            J.itVal[k] = A.get<double>(4 * L);
+            J.itXval[k] = A.get<double>(4 * L);
+            J.itVal32[k] = A.get<float>(4 * L);
+            J.itXval32[k] = A.get<float>(4 * L);
+        }
+        J.itemTotal = A.get<int>(3);
+        J.ownCnt = A.get<int>((rows + 1) * J.pcCluster);
+        J.ownPtr = A.get<int>((rows + 1) * J.pcCluster + 1);
+        J.ownFill = A.get<int>((rows + 1) * J.pcCluster);
+        J.itemPtr = A.get<int>((rows + 1) * J.pcCluster + 1);
         // FP32 copies for the mixed-precision solve
         J.val32 = A.get<float>(rows * ROW_W);
-        J.fvalP32 = A.get<float>(rows * PC_MAXE);
-        J.bvalP32 = A.get<float>(rows * PC_MAXE);
-        J.linvd32 = A.get<float>(rows);
-        J.rl32 = A.get<float>(rows);
-        J.yl32 = A.get<float>(rows);
-        J.fval32 = A.get<float>(rows * ROW_W / 2 + 1);
-        J.bval32 = A.get<float>(rows * ROW_W / 2 + 1);
         J.e32 = A.get<float>(rows);
         J.r32 = A.get<float>(rows);
         J.s32 = A.get<float>(rows);
         J.z32 = A.get<float>(rows);
         J.q32 = A.get<float>(rows);
-        J.lself = A.get<int>(rows);
-        J.yl = A.get<double>(rows);
-        J.ownCnt = A.get<int>((rows + 1) * J.pcCluster);
-        J.ownPtr = A.get<int>((rows + 1) * J.pcCluster + 1);
-        J.ownFill = A.get<int>((rows + 1) * J.pcCluster);
     }
-    if (J.pcCluster) {
+    if (J.pcCluster && !J.pcAsync) {
         J.pos = A.get<int>(rows);
         J.lcntF = A.get<int>(rows);
         J.lcntB = A.get<int>(rows);

@@ -1091,8 +1091,7 @@ struct astg_handle {
                 Cc.corrT = dCorrT;
                 launch_tilt_corr(d, Cc, dCorrT, st);
                 if (P.tilt_adaptivity) launch_adjust(d, Cc, N, dOpen, dFixed, dt, st);
-                launch_advect_scalars(d, Cc, N, dOpen, dt, st);
-                launch_advect_velocity(d, Cc, N, dt, st);
+                launch_advect(d, Cc, N, dOpen, dt, st);
                 cur = 1 - cur;
                 launch_decay(d, F[cur], st);
                 break;

@@ -292,9 +292,8 @@ void launch_dual(const Dev& d, const Fields& F, cudaStream_t st);
 void launch_adjust(const Dev& d, const Fields& cur, const Fields& nxt, uint8_t* open, uint8_t* fixedf, double dt,
                    cudaStream_t st);
 void launch_tilt_e_ghost(const Dev& d, double* te, uint32_t* tf, cudaStream_t st);
-void launch_advect_scalars(const Dev& d, const Fields& cur, const Fields& nxt, const uint8_t* open, double dt,
-                           cudaStream_t st);
-void launch_advect_velocity(const Dev& d, const Fields& cur, const Fields& nxt, double dt, cudaStream_t st);
+// scalars (with their ghosts) and velocity advected from cur into nxt
+void launch_advect(const Dev& d, const Fields& cur, const Fields& nxt, const uint8_t* open, double dt, cudaStream_t st);
 void launch_decay(const Dev& d, const Fields& F, cudaStream_t st);
 // FmmLevelSetSolver3::extrapolate of (oct, til) in place from a res^3 signed distance grid on the
 // device; scratch holds extrapolate_scratch_bytes(S); returns the nodes assigned (-1: CUDA error)

@@ -197,46 +197,62 @@ ASTG_HD inline double force_at(const Dev& d, const Fields& F, V3 p, double amb) 
     scalar_sample2(d, p, F.dO, F.dT, F.hO, F.hT, F.tf, &dv, &hv);
     return d.buoyD * dv + d.buoyT * (hv - amb);
 }
-__global__ void k_force_mac(Dev d, Fields F, const double* amb, double dt) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.S || ghost(d, s)) return;
-    if (!mac_valid(d, 2, slot_l(d, s), slot_x(d, s), slot_y(d, s), slot_z(d, s))) return;
-    double* w = F.mac + 2 * (size_t)d.S + s;
-    *w = *w + dt * force_at(d, F, mac_pos(d, 2, s), *amb);
-}
-// one thread per (tilt, slot)
-__global__ void k_force_tilt(Dev d, Fields F, const uint8_t* open, const double* amb, double dt) {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 8LL * d.S) return;
-    int s = (int)(idx >> 3), k = (int)(idx & 7);
-    if (ghost(d, s) || !open[s]) return;
-    double nf = tilt_up(k, 2) * force_at(d, F, tilt_pos(vert_pos(d, s), k, F.te[s]), *amb);
-    F.tv[(size_t)s * 8 + k] = F.tv[(size_t)s * 8 + k] + dt * nf;
-}
-// one thread per (half tilt, slot); slots the half tilt does not use get + dt * 0
-__global__ void k_force_half(Dev d, Fields F, const double* amb, double dt) {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 8LL * d.H) return;
-    int i = (int)(idx >> 3), k = (int)(idx & 7);
-    int hs = d.half[i];
-    int dir = tf_dir(F.tf[hs]);
+// the slot tilt_dir of half tilt k's face: its direction and position (q: index among its five faces, -1
+// when slot k is not one of them)
+__device__ __forceinline__ int half_face(int dir, int k) {
     int q = -1;
     for (int j = 0; j < 5; ++j)
         if (HALF_SLOT[dir][j] == k) q = j;
-    double nf = 0;
-    if (q >= 0) {
-        V3 c = vert_pos(d, hs);
-        V3 p = (q == 4) ? c : tilt_pos(c, k, F.te[hs]);
-        double tf = force_at(d, F, p, *amb);
-        V3 dv = (q == 4) ? v3(HALF_DIR_POS[k][0], HALF_DIR_POS[k][1], HALF_DIR_POS[k][2]) : tilt_up3(k);
-        nf = dot3(v3(0, 0, tf), dv);
+    return q;
+}
+// One launch for the half tilts (one thread per half tilt and slot; slots a half tilt does not use get
+// + dt * 0), the open tilts (one thread per slot and tilt) and the vertical MAC faces, in block ranges.
+// Each thread is one long chain of dependent loads and FP64 operations (the samples near level
+// transitions above all), so small grids and the few half tilts took a chain's length per launch: side by
+// side they take it once (buoyancy 0.53 -> 0.41 ms per step at 64^3 x 3, 0.33 -> 0.23 ms at 8^3 x 3).  The
+// longest chains come first.
+__global__ void k_force(Dev d, Fields F, const uint8_t* open, const double* amb, double dt) {
+    const int bH = (8 * d.H + TB - 1) / TB, bT = (int)((8LL * d.S + TB - 1) / TB);
+    int b = blockIdx.x;
+    V3 p, dv = v3(0, 0, 0);
+    double* out;
+    bool face = false;
+    if (b < bH) {
+        const int idx = b * TB + threadIdx.x;
+        if (idx >= 8 * d.H) return;
+        const int hs = d.half[idx >> 3], k = idx & 7;
+        const int q = half_face(tf_dir(F.tf[hs]), k);
+        out = F.tv + (size_t)hs * 8 + k;
+        if (q < 0) {
+            *out = *out + dt * 0.0;
+            return;
+        }
+        const V3 c = vert_pos(d, hs);
+        p = q == 4 ? c : tilt_pos(c, k, F.te[hs]);
+        dv = q == 4 ? v3(HALF_DIR_POS[k][0], HALF_DIR_POS[k][1], HALF_DIR_POS[k][2]) : tilt_up3(k);
+    } else if ((b -= bH) < bT) {
+        const long long idx = (long long)b * TB + threadIdx.x;
+        if (idx >= 8LL * d.S) return;
+        const int s = (int)(idx >> 3), k = (int)(idx & 7);
+        if (ghost(d, s) || !open[s]) return;
+        p = tilt_pos(vert_pos(d, s), k, F.te[s]);
+        dv.z = tilt_up(k, 2);
+        out = F.tv + idx;
+        face = true;
+    } else {
+        const int s = (b - bT) * TB + threadIdx.x;
+        if (s >= d.S || ghost(d, s)) return;
+        if (!mac_valid(d, 2, slot_l(d, s), slot_x(d, s), slot_y(d, s), slot_z(d, s))) return;
+        p = mac_pos(d, 2, s);
+        dv.z = 1.0;
+        out = F.mac + 2 * (size_t)d.S + s;
+        face = true;
     }
-    F.tv[(size_t)hs * 8 + k] = F.tv[(size_t)hs * 8 + k] + dt * nf;
+    const double f = force_at(d, F, p, *amb);
+    *out = *out + dt * (face ? dv.z * f : dot3(v3(0, 0, f), dv));
 }
 void launch_force(const Dev& d, const Fields& F, const uint8_t* open, const double* amb, double dt, cudaStream_t st) {
-    ASTG_LAUNCH(k_force_mac<<<nblk(d.S), TB, 0, st>>>(d, F, amb, dt));
-    ASTG_LAUNCH(k_force_tilt<<<nblk(8LL * d.S), TB, 0, st>>>(d, F, open, amb, dt));
-    if (d.H) ASTG_LAUNCH(k_force_half<<<nblk(8LL * d.H), TB, 0, st>>>(d, F, amb, dt));
+    ASTG_LAUNCH(k_force<<<nblk(8LL * d.H) + nblk(8LL * d.S) + nblk(d.S), TB, 0, st>>>(d, F, open, amb, dt));
 }
 
 // ------------------------------------------------------------------ walls and velocity ghosts
@@ -595,62 +611,76 @@ void launch_adjust(const Dev& d, const Fields& cur, const Fields& nxt, uint8_t* 
 // src/octree_omnigrid_solver3.cpp:850-914 and SemiLagrangianOctreeOmniFace3,
 // include/advection.h:195-239.  cur is the source, nxt the destination (its tilt-E is the
 // adjusted one).
-__global__ void k_adv_scalar_oct(Dev d, Fields cur, Fields nxt, double dt) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.S || ghost(d, s)) return;
-    V3 o = back_trace(d, cell_pos(d, s), dt, cur);
-    scalar_sample2(d, o, cur.dO, cur.dT, cur.hO, cur.hT, cur.tf, &nxt.dO[s], &nxt.hO[s]);
-}
-__global__ void k_adv_scalar_tilt(Dev d, Fields cur, Fields nxt, const uint8_t* open, double dt) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.S || ghost(d, s) || !open[s]) return;
-    V3 o = back_trace(d, vert_pos(d, s), dt, cur);
-    scalar_sample2(d, o, cur.dO, cur.dT, cur.hO, cur.hT, cur.tf, &nxt.dT[s], &nxt.hT[s]);
-}
-__global__ void k_adv_scalar_half(Dev d, Fields cur, Fields nxt, double dt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.H) return;
-    int hs = d.half[i];
-    V3 o = back_trace(d, vert_pos(d, hs), dt, cur);
-    scalar_sample2(d, o, cur.dO, cur.dT, cur.hO, cur.hT, cur.tf, &nxt.dT[hs], &nxt.hT[hs]);
-}
-// one thread per (axis, slot)
-__global__ void k_adv_mac(Dev d, Fields cur, Fields nxt, double dt) {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 3LL * d.S) return;
-    int a = (int)(idx / d.S), s = (int)(idx - (long long)a * d.S);
-    if (ghost(d, s)) return;
-    V3 o = back_trace(d, mac_pos(d, a, s), dt, cur);
-    nxt.mac[(size_t)a * d.S + s] = vel_sample_axis(d, o, cur, a);
-}
-// one thread per (tilt, slot)
-__global__ void k_adv_tilt(Dev d, Fields cur, Fields nxt, double dt) {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 8LL * d.S) return;
-    int s = (int)(idx >> 3), k = (int)(idx & 7);
-    if (ghost(d, s) || (nxt.tf[s] & TF_CLOSED)) return;
-    V3 o = back_trace(d, tilt_pos(vert_pos(d, s), k, nxt.te[s]), dt, cur);
-    nxt.tv[(size_t)s * 8 + k] = dot3(vel_sample(d, o, cur), tilt_up3(k));
-}
-// one thread per (half tilt, slot); unused slots are zero
-__global__ void k_adv_half(Dev d, Fields cur, Fields nxt, double dt) {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 8LL * d.H) return;
-    int i = (int)(idx >> 3), k = (int)(idx & 7);
-    int hs = d.half[i];
-    int dir = tf_dir(nxt.tf[hs]);
-    int q = -1;
-    for (int j = 0; j < 5; ++j)
-        if (HALF_SLOT[dir][j] == k) q = j;
-    double v = 0;
-    if (q >= 0) {
-        V3 c = vert_pos(d, hs);
-        V3 pos = (q == 4) ? c : tilt_pos(c, k, nxt.te[hs]);
-        V3 o = back_trace(d, pos, dt, cur);
-        V3 dv = (q == 4) ? v3(HALF_DIR_POS[k][0], HALF_DIR_POS[k][1], HALF_DIR_POS[k][2]) : tilt_up3(k);
-        v = dot3(vel_sample(d, o, cur), dv);
+//
+// One launch, in block ranges: half tilts (scalars, then one thread per half tilt and slot; unused
+// slots are zero), tilted faces (one thread per slot and tilt), tilt scalars, cell scalars, MAC faces
+// (one thread per axis and slot).  A thread is one chain of dependent gathers and FP64 operations (two
+// velocity samples of the RK2 back-trace, then the sample), up to 0.4 ms long near level transitions:
+// in launches of their own the 6 kinds took that long each, however few they were.  The longest chains
+// come first, and the back-trace's code is shared.  Advection per step 3.49 -> 2.82 ms at 64^3 x 3 and
+// 1.77 -> 0.64 ms at 8^3 x 3; bound by FP64 issue at the large size, by the chain at the small one.
+__global__ void k_advect(Dev d, Fields cur, Fields nxt, const uint8_t* open, double dt) {
+    const int bH = (d.H + TB - 1) / TB, bH8 = (8 * d.H + TB - 1) / TB, bS = (d.S + TB - 1) / TB,
+              bT = (int)((8LL * d.S + TB - 1) / TB);
+    enum { SCALAR_TILT, SCALAR_OCT, FACE, MAC } kind;
+    int b = blockIdx.x, s, k = 0;
+    V3 p, dv = v3(0, 0, 0);
+    if (b < bH) {
+        const int i = b * TB + threadIdx.x;
+        if (i >= d.H) return;
+        kind = SCALAR_TILT;
+        s = d.half[i];
+        p = vert_pos(d, s);
+    } else if ((b -= bH) < bH8) {
+        const int idx = b * TB + threadIdx.x;
+        if (idx >= 8 * d.H) return;
+        kind = FACE;
+        s = d.half[idx >> 3];
+        k = idx & 7;
+        const int q = half_face(tf_dir(nxt.tf[s]), k);
+        if (q < 0) {
+            nxt.tv[(size_t)s * 8 + k] = 0;
+            return;
+        }
+        const V3 c = vert_pos(d, s);
+        p = q == 4 ? c : tilt_pos(c, k, nxt.te[s]);
+        dv = q == 4 ? v3(HALF_DIR_POS[k][0], HALF_DIR_POS[k][1], HALF_DIR_POS[k][2]) : tilt_up3(k);
+    } else if ((b -= bH8) < bT) {
+        const long long idx = (long long)b * TB + threadIdx.x;
+        if (idx >= 8LL * d.S) return;
+        kind = FACE;
+        s = (int)(idx >> 3);
+        k = (int)(idx & 7);
+        if (ghost(d, s) || (nxt.tf[s] & TF_CLOSED)) return;
+        p = tilt_pos(vert_pos(d, s), k, nxt.te[s]);
+        dv = tilt_up3(k);
+    } else if ((b -= bT) < bS) {
+        kind = SCALAR_TILT;
+        s = b * TB + threadIdx.x;
+        if (s >= d.S || ghost(d, s) || !open[s]) return;
+        p = vert_pos(d, s);
+    } else if ((b -= bS) < bS) {
+        kind = SCALAR_OCT;
+        s = b * TB + threadIdx.x;
+        if (s >= d.S || ghost(d, s)) return;
+        p = cell_pos(d, s);
+    } else {
+        kind = MAC;
+        const long long idx = (long long)(b - bS) * TB + threadIdx.x;
+        if (idx >= 3LL * d.S) return;
+        k = (int)(idx / d.S);
+        s = (int)(idx - (long long)k * d.S);
+        if (ghost(d, s)) return;
+        p = mac_pos(d, k, s);
     }
-    nxt.tv[(size_t)hs * 8 + k] = v;
+    const V3 o = back_trace(d, p, dt, cur);
+    if (kind == MAC) nxt.mac[(size_t)k * d.S + s] = vel_sample_axis(d, o, cur, k);
+    else if (kind == FACE) nxt.tv[(size_t)s * 8 + k] = dot3(vel_sample(d, o, cur), dv);
+    else {
+        double* dd = kind == SCALAR_OCT ? nxt.dO : nxt.dT;
+        double* hh = kind == SCALAR_OCT ? nxt.hO : nxt.hT;
+        scalar_sample2(d, o, cur.dO, cur.dT, cur.hO, cur.hT, cur.tf, dd + s, hh + s);
+    }
 }
 __global__ void k_decay(Dev d, Fields F) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -660,11 +690,9 @@ __global__ void k_decay(Dev d, Fields F) {
     F.hO[s] *= d.decay;
     F.hT[s] *= d.decay;
 }
-void launch_advect_scalars(const Dev& d, const Fields& cur, const Fields& nxt, const uint8_t* open, double dt,
-                           cudaStream_t st) {
-    ASTG_LAUNCH(k_adv_scalar_oct<<<nblk(d.S), TB, 0, st>>>(d, cur, nxt, dt));
-    ASTG_LAUNCH(k_adv_scalar_tilt<<<nblk(d.S), TB, 0, st>>>(d, cur, nxt, open, dt));
-    if (d.H) ASTG_LAUNCH(k_adv_scalar_half<<<nblk(d.H), TB, 0, st>>>(d, cur, nxt, dt));
+void launch_advect(const Dev& d, const Fields& cur, const Fields& nxt, const uint8_t* open, double dt, cudaStream_t st) {
+    const int blocks = nblk(d.H) + nblk(8LL * d.H) + nblk(8LL * d.S) + 2 * nblk(d.S) + nblk(3LL * d.S);
+    ASTG_LAUNCH(k_advect<<<blocks, TB, 0, st>>>(d, cur, nxt, open, dt));
     launch_scalar_ghost(d, nxt.dO, nxt.dT, nxt.te, nxt.tf, st);
     launch_scalar_ghost(d, nxt.hO, nxt.hT, nxt.te, nxt.tf, st);
 }
@@ -679,11 +707,6 @@ __global__ void k_tilt_corr(Dev d, Fields F, double* corr) {
 }
 void launch_tilt_corr(const Dev& d, const Fields& F, double* corr, cudaStream_t st) {
     ASTG_LAUNCH(k_tilt_corr<<<nblk(d.S), TB, 0, st>>>(d, F, corr));
-}
-void launch_advect_velocity(const Dev& d, const Fields& cur, const Fields& nxt, double dt, cudaStream_t st) {
-    ASTG_LAUNCH(k_adv_mac<<<nblk(3LL * d.S), TB, 0, st>>>(d, cur, nxt, dt));
-    ASTG_LAUNCH(k_adv_tilt<<<nblk(8LL * d.S), TB, 0, st>>>(d, cur, nxt, dt));
-    if (d.H) ASTG_LAUNCH(k_adv_half<<<nblk(8LL * d.H), TB, 0, st>>>(d, cur, nxt, dt));
 }
 void launch_decay(const Dev& d, const Fields& F, cudaStream_t st) { ASTG_LAUNCH(k_decay<<<nblk(d.S), TB, 0, st>>>(d, F)); }
 

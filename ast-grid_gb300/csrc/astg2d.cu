@@ -18,10 +18,13 @@
 // and one fused advection kernel (layout adjustment, density, heat, tilted faces and MAC faces;
 // density and heat share each back-trace).
 #include <cstdint>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "astg_launch.h"
 #include "astg2d_launch.h"
+
+namespace cg = cooperative_groups;
 
 namespace astg {
 namespace g2 {
@@ -446,19 +449,33 @@ __global__ void k2_cfl(Grid2 g, const double* mx, const double* my, unsigned lon
 // multiply-subtract each and multiplies by its pivot reciprocal last -- the generic sweeps'
 // arithmetic (and the oracle's in reduce mode 1), so the result is bit-identical.
 //
-// One CTA, one thread per column (column x = lane x % 32 of warp x / 32), one block barrier per
-// diagonal.  A column's own previous result is the neighbour below (forward) or above (backward)
-// and stays in a register; the neighbour to the left / right is the adjacent lane's previous
-// result (a warp shuffle), across a warp boundary a shared-memory slot per warp and step parity.
-// The per-cell records, the residual and the results are stored diagonal-major (cell (x, y) at
-// x + (x + y) * nx), so every step's accesses are contiguous across a warp; they are loaded WAVE_PF
-// steps ahead.  A second kernel returns the cells' result to the system's order.  Each step's
-// critical path is three dependent FP64 operations (~60 cycles each on this GPU) plus a shuffle
-// and the barrier.  (A barrier-free form with per-warp progress counters measured 1.5x slower:
-// its per-step handshake and fences cost more than the barrier.)
-constexpr int WAVE_PF = 4;
+// One warp per 32 columns, each in a CTA of its own, the CTAs one cluster.  A lane owns a column and
+// runs one row behind the lane to its left, so the neighbour below / above is its own previous result
+// (a register) and the neighbour to the left / right the adjacent lane's (a shuffle), with no barrier
+// anywhere.  Between warps, the boundary lane stores each result into the next CTA's shared memory
+// (one slot per row, empty until then: a signalling-NaN bit pattern that no arithmetic produces); the
+// reader falls a few steps behind and from then on finds the value waiting.  The per-cell records, the
+// residual and the results are stored by the warp's diagonals (Proj::wave), so WAVE_CHUNK steps of
+// them are one contiguous piece each, which bulk copies bring into shared memory WAVE_STAGES chunks
+// ahead (copies by the lanes of a second warp cost the sweep 30 to 100 cycles a step): the sweeping
+// warp has little else to issue than its chain.  An absent neighbour has the entry 0 and the result 0,
+// and so have the slots outside the grid: nothing is selected on the way from one step to the next.
+//
+// What bounds it: the chain, a shuffle and three dependent FP64 operations per diagonal (~280 cycles
+// with the records and results of the group; four more operations in the backward sweep where tilts
+// are open), over the grid's nx + ny diagonals and ~5 more per warp.  With all columns in one CTA the
+// SM's one FP64 pipe (a warp instruction per ~17 cycles, predicated-off ones included) and a block
+// barrier per diagonal made a step ~650 cycles.  Per application at 192 x 384 on GB300: 360 -> 172 us;
+// whole frames, 213 -> 117 ms there and 7.7 -> 5.9 ms at 45 x 83.
+constexpr int WAVE_STAGES = 3;
 constexpr int WAVE_MAX_NX = 512;
-constexpr int WAVE_MAX_W = WAVE_MAX_NX / 32;
+constexpr int WAVE_THREADS = 256;  // warp 0 sweeps, a thread of warp 1 copies, all do the tilt rows
+// one chunk's records: WAVE_CHUNK lines of wRecF or wRecB, of wR or wZ, of wTl and of wTz
+constexpr int WAVE_VAL = WAVE_CHUNK * 1024, WAVE_TL = WAVE_VAL + WAVE_CHUNK * 256, WAVE_TZ = WAVE_TL + WAVE_CHUNK * 1024;
+constexpr int WAVE_STAGE = WAVE_TZ + WAVE_CHUNK * 1024;
+constexpr int WAVE_RING = WAVE_STAGES * WAVE_STAGE;
+constexpr int WAVE_PAD = 48;       // edge slots before row 0 and after row ny - 1
+constexpr int WAVE_MAX_NY = (224 * 1024 - WAVE_RING) / 8 - 2 * WAVE_PAD;
 
 // records of the factorised system for the wavefront kernel (one thread per row)
 __global__ void k2_wave_gather(Proj P, const int* vIdx) {
@@ -482,178 +499,285 @@ __global__ void k2_wave_gather(Proj P, const int* vIdx) {
         }
         return;
     }
-    const int x = r % nx, y = r / nx, j = x + (x + y) * nx;  // diagonal-major slot
+    const int x = r % nx, y = r / nx, j = wave_slot(x, y, ny), line = j >> 5, lane = j & 31;
     const int corner[4] = {vIdx[x + y * (nx + 1)], vIdx[x + 1 + y * (nx + 1)], vIdx[x + (y + 1) * (nx + 1)],
                            vIdx[x + 1 + (y + 1) * (nx + 1)]};
     double lb = 0, ll = 0, lr = 0, la = 0;
-    unsigned f = 0;
-    for (int k = 0; k < 4; ++k) {
-        P.wTt[4 * j + k] = -1;
-        P.wTl[4 * j + k] = 0;
-    }
+    double tl[4] = {0, 0, 0, 0};
+    bool open = false;
     for (int q = q0; q < q1; ++q) {
         const int col = P.col[q];
-        if (col == r - nx) { lb = P.Lv[P.tpos[q]]; f |= 1; }
-        else if (col == r - 1) { ll = P.Lv[P.tpos[q]]; f |= 2; }
-        else if (col == r + 1) { lr = P.Lv[q]; f |= 4; }
-        else if (col == r + nx) { la = P.Lv[q]; f |= 8; }
+        if (col == r - nx) lb = P.Lv[P.tpos[q]];
+        else if (col == r - 1) ll = P.Lv[P.tpos[q]];
+        else if (col == r + 1) lr = P.Lv[q];
+        else if (col == r + nx) la = P.Lv[q];
         else if (col >= nc) {
             for (int k = 0; k < 4; ++k)
                 if (corner[k] == col) {
-                    P.wTt[4 * j + k] = col;
-                    P.wTl[4 * j + k] = P.Lv[q];
-                    f |= 16u << k;
+                    tl[k] = P.Lv[q];
+                    open = true;
                 }
         }
     }
-    const double inv = P.invdiag[r], fb = __longlong_as_double((long long)f);
-    P.wRecF[2 * j] = make_double2(lb, ll);
-    P.wRecF[2 * j + 1] = make_double2(inv, fb);
-    P.wRecB[2 * j] = make_double2(lr, la);
-    P.wRecB[2 * j + 1] = make_double2(inv, fb);
-}
-
-constexpr unsigned WAVE_NONE = 0x80000000u;  // no cell in this column on this diagonal
-struct WStep {
-    double v, l0, l1, inv;
-    unsigned f;
-};
-// one slot's record; WAVE_NONE when the column has no cell on the diagonal (then nothing is
-// computed: a warp with no cell on a diagonal issues no FP64 work there)
-__device__ __forceinline__ void wload(const double2* rec, const double* val, int j, bool on, WStep& s) {
-    if (!on) {
-        s.f = WAVE_NONE;
-        return;
+    const double inv = P.invdiag[r];
+    P.wRecF[line * 64 + lane] = make_double2(lb, ll);
+    P.wRecF[line * 64 + 32 + lane] = make_double2(inv, 0);
+    P.wRecB[line * 64 + lane] = make_double2(lr, la);
+    P.wRecB[line * 64 + 32 + lane] = make_double2(inv, __longlong_as_double(open));
+    for (int k = 0; k < 4; ++k) {
+        P.wTl[line * 128 + k * 32 + lane] = tl[k];
+        P.wTz[line * 128 + k * 32 + lane] = 0;
     }
-    const double2 a = rec[2 * j], b = rec[2 * j + 1];
-    s.v = val[j];
-    s.l0 = a.x;
-    s.l1 = a.y;
-    s.inv = b.x;
-    s.f = (unsigned)__double_as_longlong(b.y);
+    if (open) P.wTf[line / WAVE_CHUNK] = 1;
 }
 
-// the cells' result from diagonal-major order to the system's
-__global__ void k2_wave_unskew(Proj P, double* z) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nx = P.wnx;
-    if (*P.done || i >= nx * P.wny) return;
-    const int x = i % nx;
-    z[i] = P.wZ[x + (x + i / nx) * nx];
+constexpr unsigned long long WAVE_EMPTY = 0x7FF4DEADBEEF0001ull;
+constexpr long long WAVE_SPIN_LIMIT = 1LL << 22;
+__device__ __forceinline__ double2 wave_ld2(uint32_t a) {
+    double2 v;
+    asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ double wave_ld1(uint32_t a) {
+    double v;
+    asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool wave_empty(double v) { return __double2hiint(v) == (int)(WAVE_EMPTY >> 32); }
+// waits for the phase of `parity`; false past the limit (status), or, given a status, once any wait
+// has given up
+__device__ __forceinline__ bool wave_wait(uint32_t bar, int parity, int* status) {
+    for (long long it = 1; it <= WAVE_SPIN_LIMIT; ++it) {
+        int ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.s32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+        if (status && (it & 255) == 0 && *(volatile int*)status != 0) return false;
+    }
+    if (status) atomicCAS(status, 0, DS_WAIT_TIMEOUT);
+    return false;
+}
+// one warp's columns
+struct WaveWarp {
+    uint32_t ring, bars;       // records; full[WAVE_STAGES] then freed[WAVE_STAGES]
+    int x, line0, chunks, g0;  // this lane's column; the warp's first line; its chunks; chunks of earlier sweeps
+};
+// the copying thread: the chunks of a sweep in its order, then their completion (nothing is in flight
+// when it returns, also when the sweep gave up)
+template <bool FWD>
+__device__ __forceinline__ void wave_copy(const Proj& P, const WaveWarp& W) {
+    int issued = 0;
+    for (int c = 0; c < W.chunks; ++c, ++issued) {
+        const int g = W.g0 + c, s = g % WAVE_STAGES;
+        if (g >= WAVE_STAGES && !wave_wait(W.bars + 8 * (WAVE_STAGES + s), (g / WAVE_STAGES - 1) & 1, P.wStatus)) break;
+        const long long line = W.line0 + (FWD ? c : W.chunks - 1 - c) * WAVE_CHUNK;
+        const bool tilts = !FWD && P.wTf[line / WAVE_CHUNK] != 0;
+        const uint32_t dst = W.ring + s * WAVE_STAGE, bar = W.bars + 8 * s;
+        auto bulk = [&](uint32_t to, const void* src, int bytes) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to), "l"(src),
+                         "r"(bytes), "r"(bar)
+                         : "memory");
+        };
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tilts ? WAVE_STAGE : WAVE_TL) : "memory");
+        bulk(dst, (FWD ? P.wRecF : P.wRecB) + line * 64, WAVE_CHUNK * 1024);
+        bulk(dst + WAVE_VAL, (FWD ? P.wR : P.wZ) + line * 32, WAVE_CHUNK * 256);
+        if (tilts) {
+            bulk(dst + WAVE_TL, P.wTl + line * 128, WAVE_CHUNK * 1024);
+            bulk(dst + WAVE_TZ, P.wTz + line * 128, WAVE_CHUNK * 1024);
+        }
+    }
+    for (int c = issued > WAVE_STAGES ? issued - WAVE_STAGES : 0; c < issued; ++c) {
+        const int g = W.g0 + c;
+        wave_wait(W.bars + 8 * (g % WAVE_STAGES), (g / WAVE_STAGES) & 1, nullptr);
+    }
 }
 
-__global__ void __launch_bounds__(WAVE_MAX_NX) k2_precond_wave(Proj P, const double* r, double* z) {
-    __shared__ double edge[2][WAVE_MAX_W];  // per step parity: each warp's boundary value
+// One sweep over the warp's lines, upwards (forward) or downwards (backward).  The boundary lane (0
+// forward, 31 backward) takes its neighbour's results from `edge` (by row; the slots outside the
+// grid hold 0, and so do all of them in the warp that has no such neighbour: no step checks the
+// range), the opposite lane stores its own into `peer` (0: none).  The warp issues in order and pays
+// 20 to 30 cycles for each load or store among a step's FP64 operations, so these stand together:
+// once per WAVE_GROUP steps, the next group's records and edge values and this group's results.
+constexpr int WAVE_GROUP = 2;
+struct WaveGroup {
+    double2 l[WAVE_GROUP], iv[WAVE_GROUP];
+    double v[WAVE_GROUP], edge[WAVE_GROUP];
+};
+template <bool FWD>
+__device__ __forceinline__ void wave_sweep(const Proj& P, const WaveWarp& W, uint32_t edge, uint32_t peer) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sd = FWD ? 1 : -1;
+    const unsigned bound = W.x < P.wnx ? P.wny : 0;
+    const bool first = lane == (FWD ? 0 : 31), writer = peer != 0 && lane == (FWD ? 31 : 0);
+    const int start = FWD ? 0 : W.chunks * WAVE_CHUNK - 1;  // the sweep's first line
+    int y = start - lane;                                   // this lane's row
+    uint32_t ea = edge + 8 * (start - (FWD ? 0 : 31));  // the boundary lane's row
+    uint32_t pa = peer + 8 * y;
+    double* out = P.wZ + (W.line0 + start) * 32LL + lane;
+    double prev = 0;  // this column's last result
+    constexpr int G = WAVE_GROUP;
+    WaveGroup cur, nxt;
+    auto loadEdge = [&](WaveGroup& q) {
+#pragma unroll
+        for (int k = 0; k + 1 < G; k += 2) {
+            const double2 a = wave_ld2(FWD ? ea + 8 * k : ea - 8 - 8 * k);
+            q.edge[k] = FWD ? a.x : a.y;
+            q.edge[k + 1] = FWD ? a.y : a.x;
+        }
+    };
+    auto load = [&](WaveGroup& q, uint32_t stage, int h) {
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            const int i = FWD ? h * G + k : WAVE_CHUNK - 1 - h * G - k;
+            q.l[k] = wave_ld2(stage + i * 1024 + lane * 16);
+            q.iv[k] = wave_ld2(stage + i * 1024 + 512 + lane * 16);
+            q.v[k] = wave_ld1(stage + WAVE_VAL + i * 256 + lane * 8);
+        }
+    };
+    auto empty = [&](const WaveGroup& q) {  // the same slots for all lanes
+        bool e = false;
+#pragma unroll
+        for (int k = 0; k < G; ++k) e = e || wave_empty(q.edge[k]);
+        return e;
+    };
+    auto full = [&](int g) {
+        wave_wait(W.bars + 8 * (g % WAVE_STAGES), (g / WAVE_STAGES) & 1, P.wStatus);
+        __syncwarp();
+        return W.ring + (uint32_t)(g % WAVE_STAGES) * WAVE_STAGE;
+    };
+    uint32_t stage = full(W.g0);
+    load(nxt, stage, 0);
+    loadEdge(nxt);
+#pragma unroll 1
+    for (int c = 0; c < W.chunks; ++c) {
+        const int g = W.g0 + c;
+        uint32_t next = stage;
+#pragma unroll
+        for (int h = 0; h < WAVE_CHUNK / G; ++h) {
+            for (long long it = 1; empty(nxt); ++it) {
+                loadEdge(nxt);
+                if ((it & 255) == 0) {
+                    if (it > WAVE_SPIN_LIMIT) atomicCAS(P.wStatus, 0, DS_WAIT_TIMEOUT);
+                    if (*(volatile int*)P.wStatus != 0)
+                        for (int k = 0; k < G; ++k) nxt.edge[k] = 0;
+                }
+            }
+            __syncwarp();
+            cur = nxt;
+            ea += 8 * G * sd;
+            if (h + 1 < WAVE_CHUNK / G) {
+                load(nxt, stage, h + 1);
+            } else if (c + 1 < W.chunks) {
+                next = full(g + 1);
+                load(nxt, next, 0);
+            }
+            loadEdge(nxt);
+            double res[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                // forward: below (own), then left; backward: right, then above (own), then the corner tilts
+                double side = FWD ? __shfl_up_sync(FULL, prev, 1) : __shfl_down_sync(FULL, prev, 1);
+                double acc = FWD ? fma(-cur.l[k].x, prev, cur.v[k]) : cur.v[k];
+                if (first) side = cur.edge[k];
+                acc = fma(FWD ? -cur.l[k].y : -cur.l[k].x, side, acc);
+                if (!FWD) acc = fma(-cur.l[k].y, prev, acc);
+                // the tilts' entries and results (zero where closed); the forward records have none,
+                // but the branch keeps the group's loads and stores out of the chain there too
+                // (without it 320 cycles a step instead of 280)
+                const int open = __any_sync(FULL, __double2loint(cur.iv[k].y)) ? 4 : 0;
+                const uint32_t tl = stage + WAVE_TL + (WAVE_CHUNK - 1 - h * G - k) * 1024 + lane * 8;
+#pragma unroll 1
+                for (int q = 0; q < open; ++q) acc = fma(-wave_ld1(tl + q * 256), wave_ld1(tl + q * 256 + (WAVE_TZ - WAVE_TL)), acc);
+                res[k] = prev = acc * cur.iv[k].x;
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                asm volatile(
+                    "{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n setp.ne.b32 q, %4, 0;\n"
+                    " @q st.shared::cluster.f64 [%1], %2;\n @p st.global.f64 [%0], %2;\n}" ::"l"(out + sd * 32 * k),
+                    "r"(pa + 8 * sd * k), "d"(res[k]), "r"((int)((unsigned)(y + sd * k) < bound)), "r"((int)writer)
+                    : "memory");
+            }
+            out += sd * 32 * G;
+            pa += 8 * sd * G;
+            y += sd * G;
+        }
+        __syncwarp();
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(W.bars + 8 * (WAVE_STAGES + g % WAVE_STAGES)) : "memory");
+        stage = next;
+    }
+}
+// z: the tilt rows' results; the cells' stay in wZ
+__global__ void __launch_bounds__(WAVE_THREADS, 1) k2_precond_wave(Proj P, const double* r, double* z) {
+    extern __shared__ __align__(16) unsigned char wave_smem[];
+    __shared__ __align__(8) unsigned long long bars[2 * WAVE_STAGES];
+    cg::cluster_group cl = cg::this_cluster();
     if (*P.done) return;
     const int nx = P.wnx, ny = P.wny, nc = nx * ny, n = *P.nDof;
-    const int D = nx + ny - 1;
-    const int x = threadIdx.x, lane = x & 31, w = x >> 5, W = blockDim.x >> 5;
-    const bool mine = x < nx;  // lanes past the last column only take part in the exchanges
-    const unsigned FULL = 0xffffffffu;
-    WStep A[WAVE_PF], B[WAVE_PF];
-
-    // ---- forward over the cells: step d visits slot x + d * nx, the cell (x, d - x).  The update
-    // from the cell below (this column's previous result) is applied before the barrier that ends
-    // the previous step; the one from the left needs the neighbouring column's previous result
-    // (shuffle, or the boundary slot of the warp to the left for lane 0).
-    double zb = 0;  // this column's last result
-    double t = 0;   // the current slot's accumulator after the update from below
-    auto fload = [&](WStep* S, int d0) {
-#pragma unroll
-        for (int s = 0; s < WAVE_PF; ++s) {
-            const int d = d0 + s, y = d - x;
-            wload(P.wRecF, P.wR, x + d * nx, mine && y >= 0 && y < ny, S[s]);
-        }
+    const int rank = cl.block_rank(), nb = cl.num_blocks(), x0 = 32 * rank;
+    double* e = reinterpret_cast<double*>(wave_smem + WAVE_RING);
+    WaveWarp W;
+    W.ring = (uint32_t)__cvta_generic_to_shared(wave_smem);
+    W.bars = (uint32_t)__cvta_generic_to_shared(bars);
+    W.x = x0 + (threadIdx.x & 31);
+    W.line0 = rank * wave_lines(ny);
+    W.chunks = (ny + min(31, nx - 1 - x0) + WAVE_CHUNK - 1) / WAVE_CHUNK;  // up to the last line with a cell
+    W.g0 = 0;
+    const uint32_t edge = W.ring + WAVE_RING + 8 * WAVE_PAD;  // row 0
+    auto peer = [&](int q, uint32_t mine) {
+        uint32_t m = 0;
+        if (q >= 0 && q < nb) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(mine), "r"(q));
+        return m;
     };
-    auto below = [&](const WStep& c) {  // (x, y - 1)
-        return (!(c.f & WAVE_NONE) && (c.f & 1)) ? fma(-c.l0, zb, c.v) : c.v;
+    auto clear = [&](bool neighbour, int row0) {  // row 0 at slot row0
+        for (int i = threadIdx.x; i < ny + 2 * WAVE_PAD; i += blockDim.x)
+            e[i] = neighbour && i >= row0 && i < ny + row0 ? __longlong_as_double((long long)WAVE_EMPTY) : 0.0;
     };
-    auto fstep = [&](const WStep& c, const WStep& nxt, int d) {
-        const int cur = d & 1, prv = cur ^ 1;
-        double zl = __shfl_up_sync(FULL, zb, 1);
-        const double ze = edge[prv][w > 0 ? w - 1 : 0];
-        if (lane == 0) zl = ze;
-        if (!(c.f & WAVE_NONE)) {
-            double acc = (c.f & 2) ? fma(-c.l1, zl, t) : t;  // (x - 1, y)
-            acc = acc * c.inv;
-            P.wZ[x + d * nx] = acc;
-            zb = acc;
-        }
-        if (lane == 31) edge[cur][w] = zb;
-        t = below(nxt);
-        __syncthreads();
-    };
-    fload(A, 0);
-    t = below(A[0]);
-    for (int g = 0; g < D; g += 2 * WAVE_PF) {
-        fload(B, g + WAVE_PF);
-#pragma unroll
-        for (int s = 0; s < WAVE_PF; ++s)
-            if (g + s < D) fstep(A[s], s + 1 < WAVE_PF ? A[s + 1] : B[0], g + s);
-        fload(A, g + 2 * WAVE_PF);
-#pragma unroll
-        for (int s = 0; s < WAVE_PF; ++s)
-            if (g + WAVE_PF + s < D) fstep(B[s], s + 1 < WAVE_PF ? B[s + 1] : A[0], g + WAVE_PF + s);
+    clear(rank > 0, WAVE_PAD);
+    if (threadIdx.x == 32) {
+        for (int i = 0; i < 2 * WAVE_STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(W.bars + 8 * i) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-
-    // ---- tilt rows: forward (their four cells), then their backward step (no upper entries)
-    for (int tr = nc + x; tr < n; tr += blockDim.x) {
+    cl.sync();  // every CTA is running and its edge is empty
+    if (threadIdx.x < 32) wave_sweep<true>(P, W, edge, peer(rank + 1, edge));
+    else if (threadIdx.x == 32) wave_copy<true>(P, W);
+    __syncwarp();
+    __threadfence();
+    cl.sync();
+    clear(rank + 1 < nb, WAVE_PAD + 1);
+    // (rows one slot on: a group's four rows, read as two aligned pairs, then start at an odd row)
+    // tilt rows: forward (their four cells), then their backward step (no upper entries); the result
+    // also goes to the four cells' records for the backward sweep
+    for (int tr = nc + rank * blockDim.x + threadIdx.x; tr < n; tr += nb * blockDim.x) {
         const int i = tr - nc;
         double acc = r[tr];
+        int slot[4];
         for (int k = 0; k < 4; ++k) {
             const int c = P.wTc[4 * i + k];
-            if (c >= 0) acc = fma(-P.wTv[4 * i + k], P.wZ[c % nx + (c % nx + c / nx) * nx], acc);
+            slot[k] = c >= 0 ? wave_slot(c % nx, c / nx, ny) : -1;
+            if (c >= 0) acc = fma(-P.wTv[4 * i + k], __ldcg(P.wZ + slot[k]), acc);
         }
         const double inv = P.invdiag[tr];
         acc = acc * inv;
-        z[tr] = acc * inv;
+        acc = acc * inv;
+        z[tr] = acc;
+        for (int k = 0; k < 4; ++k)  // the tilt is corner 3 - k of its k-th cell
+            if (slot[k] >= 0) P.wTz[(slot[k] >> 5) * 128 + (3 - k) * 32 + (slot[k] & 31)] = acc;
     }
-    __syncthreads();
-
-    // ---- backward over the cells: step s visits diagonal D - 1 - s; the update from the right
-    // (neighbouring column, shuffle or boundary slot) comes first, then the one from above (this
-    // column's previous result), then the corner tilts
-    double za = 0;
-    auto bload = [&](WStep* S, int s0) {
-#pragma unroll
-        for (int s = 0; s < WAVE_PF; ++s) {
-            const int d = D - 1 - (s0 + s), y = d - x;
-            wload(P.wRecB, P.wZ, x + d * nx, mine && y >= 0 && y < ny, S[s]);
-        }
-    };
-    auto bstep = [&](const WStep& c, int st) {
-        const int cur = st & 1, prv = cur ^ 1;
-        double zr = __shfl_down_sync(FULL, za, 1);
-        const double ze = edge[prv][w + 1 < W ? w + 1 : w];
-        if (lane == 31) zr = ze;
-        if (!(c.f & WAVE_NONE)) {
-            double acc = c.v;
-            if (c.f & 4) acc = fma(-c.l0, zr, acc);  // (x + 1, y)
-            if (c.f & 8) acc = fma(-c.l1, za, acc);  // (x, y + 1)
-            const int j = x + (D - 1 - st) * nx;
-            if (c.f & 0xf0u) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (c.f & (16u << k)) acc = fma(-P.wTl[4 * j + k], z[P.wTt[4 * j + k]], acc);
-            }
-            acc = acc * c.inv;
-            P.wZ[j] = acc;  // in place: this slot's forward value was loaded steps ago
-            za = acc;
-        }
-        if (lane == 0) edge[cur][w] = za;
-        __syncthreads();
-    };
-    bload(A, 0);
-    for (int g = 0; g < D; g += 2 * WAVE_PF) {
-        bload(B, g + WAVE_PF);
-#pragma unroll
-        for (int s = 0; s < WAVE_PF; ++s)
-            if (g + s < D) bstep(A[s], g + s);
-        bload(A, g + 2 * WAVE_PF);
-#pragma unroll
-        for (int s = 0; s < WAVE_PF; ++s)
-            if (g + WAVE_PF + s < D) bstep(B[s], g + WAVE_PF + s);
+    __threadfence();
+    asm volatile("fence.proxy.async;" ::: "memory");  // wZ and wTz are read by bulk copies
+    cl.sync();
+    W.g0 = W.chunks;
+    if (threadIdx.x < 32) wave_sweep<false>(P, W, edge + 8, peer(rank - 1, edge + 8));
+    else if (threadIdx.x == 32) {
+        asm volatile("fence.proxy.async;" ::: "memory");
+        wave_copy<false>(P, W);
     }
+    __syncwarp();
+    cl.sync();  // no CTA leaves while a neighbour may still store into its edge
 }
 
 }  // namespace g2
@@ -704,16 +828,46 @@ void launch2_cfl(const Grid2& g, const Fields2& F, unsigned long long* out, cuda
 }
 
 void launch2_wave_gather(const Proj& P, const int* vIdx, int rows, cudaStream_t st) {
+    cudaMemsetAsync(P.wTf, 0, sizeof(int) * (wave_slots(P.wnx, P.wny) / (32 * WAVE_CHUNK)), st);
     ASTG_LAUNCH(k2_wave_gather<<<nblk2(rows), TB2, 0, st>>>(P, vIdx));
 }
-void launch_precond_wave(const Proj& P, const double* r, double* z, cudaStream_t st) {
-    const int threads = (P.wnx + 31) / 32 * 32;
-    ASTG_LAUNCH(k2_precond_wave<<<1, threads, 0, st>>>(P, r, z));
-    ASTG_LAUNCH(k2_wave_unskew<<<nblk2((long long)P.wnx * P.wny), TB2, 0, st>>>(P, z));
+static size_t wave_smem_bytes(int ny) { return (size_t)WAVE_RING + 8 * (size_t)(ny + 2 * WAVE_PAD); }
+static void wave_config(int nx, int ny, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at) {
+    const int ctas = (nx + 31) / 32;
+    cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(WAVE_THREADS);
+    cfg.dynamicSmemBytes = wave_smem_bytes(ny);
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
 }
-// the wavefront kernel takes up to WAVE_MAX_NX columns; its diagonal-major slots use 32-bit indices
+void launch_precond_wave(const Proj& P, const double* r, double* z, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    wave_config(P.wnx, P.wny, st, cfg, at);
+    count_launch();
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k2_precond_wave, P, r, z);
+    if (e != cudaSuccess) g_cluster_error = e;
+}
+// The wavefront kernel takes up to WAVE_MAX_NX columns (16 CTAs of 32) and as many rows as fit a
+// CTA's shared memory; its slots use 32-bit indices.  Wider and taller grids take the generic sweeps.  Call with the device current.
 bool wave_supported(int nx, int ny) {
-    return nx >= 2 && nx <= WAVE_MAX_NX && (long long)nx * (nx + ny - 1) * 4 < (1LL << 31);
+    if (nx < 2 || nx > WAVE_MAX_NX || ny > WAVE_MAX_NY || wave_slots(nx, ny) * 4 >= (1LL << 31)) return false;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    wave_config(nx, ny, nullptr, cfg, at);
+    int nc = 0;
+    const bool ok =
+        cudaFuncSetAttribute(k2_precond_wave, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(k2_precond_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wave_smem_bytes(WAVE_MAX_NY)) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&nc, k2_precond_wave, &cfg) == cudaSuccess && nc > 0;
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 }  // namespace astg

@@ -139,14 +139,15 @@ struct astg2_handle {
         if (useWave) {
             J.wnx = nx;
             J.wny = ny;
-            const long long skew = (long long)nx * (nx + ny - 1);  // diagonal-major slots
+            const long long skew = wave_slots(nx, ny);
             J.wRecF = dalloc<double2>(2 * skew);
             J.wRecB = dalloc<double2>(2 * skew);
             J.wR = dalloc<double>(skew);
             J.wZ = dalloc<double>(skew);
             J.wStatus = status;
-            J.wTt = dalloc<int>(4 * skew);
             J.wTl = dalloc<double>(4 * skew);
+            J.wTz = dalloc<double>(4 * skew);
+            J.wTf = dalloc<int>(skew / (32 * WAVE_CHUNK));
             J.wTc = dalloc<int>(4 * nv());
             J.wTv = dalloc<double>(4 * nv());
         }
@@ -179,7 +180,7 @@ struct astg2_handle {
         select_preconditioner(J, n);
         launch2_assemble(g, d, C, vIdx, J, dt, st);
         bool mixed = precision == ASTG_MIXED && J.pcActive32;
-        // FP64 solves take the wavefront sweeps (one CTA along the anti-diagonals); the mixed form
+        // FP64 solves take the wavefront sweeps (along the anti-diagonals); the mixed form
         // keeps the FP32 fused preconditioner
         J.wave = (useWave && !mixed) ? 1 : 0;
         if (J.wave) J.pcActive = 0;

@@ -171,27 +171,33 @@ struct Proj {
     int tolAbsolute; // 1: the PCG stops at |r|_inf <= tol (the std::vector PCGSolver::solve overload,
                      // include/pcgsolver/pcg_solver.h:302-363); 0: at tol * |b|_inf
     // wavefront form of the MIC(0) sweeps on a uniform 2-D grid (cells x + y * wnx first, then one
-    // row per open tilt), astg2d.cu.  Per cell, diagonal-major (cell (x, y) at j = x + (x + y) * wnx,
-    // wnx * (wnx + wny - 1) slots), two double2 each:
-    // wRecF = (L to the cell below, L to the cell on the left), (pivot reciprocal, flags);
-    // wRecB = (L from the cell on the right, L from the cell above), (pivot reciprocal, flags); the
-    // flags (an integer in the bits of a double) are 1 below, 2 left, 4 right, 8 above and 16 << k
-    // for corner tilt k of (x, y), (x + 1, y), (x, y + 1), (x + 1, y + 1).  wTt / wTl: those tilts'
-    // rows and entries (4 per cell); wTc / wTv: each tilt row's cells and entries, ascending.
-    // wR: the residual of the cells in the same order (written by the PCG's update), wZ: the
-    // sweeps' result of the cells in that order.
+    // row per open tilt), astg2d.cu.  A warp takes 32 columns; its diagonals are lines of 32 lanes,
+    // wave_lines(ny) of them per warp (cell (x, y) in line y + x % 32, wave_slot; the other slots hold
+    // zeros).  Per line: wRecF, 32 x (L to the cell below, L to the cell on the left), then
+    // 32 x (pivot reciprocal, 0); wRecB, 32 x (L from the cell on the right, L from the cell above),
+    // then 32 x (pivot reciprocal, 1 where a corner tilt is open, an integer in the bits of a double);
+    // wTl, 32 entries for each corner tilt of (x, y), (x + 1, y), (x, y + 1), (x + 1, y + 1); wTz,
+    // those tilts' results of the current application in the same order; wR, the residual (written by
+    // the PCG's update); wZ, the cells' result.  wTf: per 8 lines, any open tilt.
+    // wTc / wTv: each tilt row's cells and entries, ascending.
     int wave;        // 1: precond runs the wavefront kernel
     int wnx, wny;
     double2* wRecF;
     double2* wRecB;
     double* wR;
     double* wZ;
-    int* wTt;
     double* wTl;
+    double* wTz;
+    int* wTf;
     int* wTc;
     double* wTv;
     int* wStatus;    // device status word for wait time-outs
 };
+
+constexpr int WAVE_CHUNK = 8;  // lines copied at a time
+__host__ __device__ inline int wave_lines(int ny) { return (ny + 31 + WAVE_CHUNK - 1) / WAVE_CHUNK * WAVE_CHUNK; }
+__host__ __device__ inline long long wave_slots(int nx, int ny) { return (nx + 31LL) / 32 * 32 * wave_lines(ny); }
+__host__ __device__ inline int wave_slot(int x, int y, int ny) { return ((x >> 5) * wave_lines(ny) + y + (x & 31)) * 32 + (x & 31); }
 
 void launch_source(const Dev& d, const Fields& F, cudaStream_t st);
 void launch_scalar_ghost(const Dev& d, double* oct, double* til, const double* te, const uint32_t* tf, cudaStream_t st);

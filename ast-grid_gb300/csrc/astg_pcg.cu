@@ -1980,17 +1980,38 @@ __global__ void k_to_level_order(Proj P, const double* r) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *P.nDof) P.rl[P.pos[i]] = r[i];
 }
-// the residual of a cell row in the wavefront preconditioner's diagonal-major order (Proj::wave)
+// the residual of a cell row in the wavefront preconditioner's order (Proj::wave)
 __device__ __forceinline__ void wave_put_r(const Proj& P, int i, double ri) {
     const int nx = P.wnx;
-    if (i < nx * P.wny) {
-        const int x = i % nx;
-        P.wR[x + (x + i / nx) * nx] = ri;
-    }
+    if (i < nx * P.wny) P.wR[wave_slot(i % nx, i / nx, P.wny)] = ri;
 }
 __global__ void k_to_wave_order(Proj P, const double* r) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *P.nDof) wave_put_r(P, i, r[i]);
+}
+// z . r in the fixed tree's order after the wavefront preconditioner, whose cells' result is in its
+// own order: brought into the system's on the way.  (Written by the sweep itself, a step's 32 rows
+// would be 32 separate sectors on the one warp that the sweep waits for: 100 cycles a step.)
+__global__ void k_tree_dot_wave(Proj P, double* z, const double* r, double* part) {
+    grid_dep_wait();
+    __shared__ double sh[RED_LANES];
+    if (*P.done) return;
+    const int n = *P.nDof, nx = P.wnx, nc = nx * P.wny;
+    const long long base = (long long)blockIdx.x * RED_CHUNK + threadIdx.x;
+    if (base - threadIdx.x >= n) return;
+    double acc = 0;
+#pragma unroll
+    for (int k = 0; k < RED_PER_LANE; ++k) {
+        const long long i = base + (long long)RED_LANES * k;
+        if (i < n) {
+            double zi;
+            if (i < nc) z[i] = zi = P.wZ[wave_slot((int)i % nx, (int)i / nx, P.wny)];
+            else zi = z[i];
+            acc = fma(zi, r[i], acc);
+        }
+    }
+    const double s = block_tree(acc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 __global__ void k_zero_vec(double* a, const int* nptr) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2395,6 +2416,7 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
     if (P.wave) ASTG_LAUNCH(k_to_wave_order<<<nblk(maxRows), TB, 0, st>>>(P, r));
     precond(d, P, r, z, epoch, st, prof);
     if (P.refOrder) launch_dot_ref(z, r, P.nDof, P.part, st);
+    else if (P.wave) ASTG_LAUNCH(k_tree_dot_wave<<<chunks, RED_LANES, 0, st>>>(P, z, r, P.part));
     else ASTG_LAUNCH(k_tree_dot<<<chunks, RED_LANES, 0, st>>>(z, r, P.nDof, P.part));
     ASTG_LAUNCH(k_pcg_start<<<1, RED_LANES, 0, st>>>(P, P.part, tolFactor));
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(z, s, P.nDof));
@@ -2413,6 +2435,7 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
             launch_pdl(k_check, 1, 1, st, P, maxIter);
             precond(d, P, r, z, epoch, st, pf);
             if (P.refOrder) launch_dot_ref(z, r, P.nDof, P.part, st);
+            else if (P.wave) launch_pdl(k_tree_dot_wave, chunks, RED_LANES, st, P, z, r, P.part);
             else launch_pdl(k_tree_dot, chunks, RED_LANES, st, z, r, P.nDof, P.part);
             launch_pdl(k_beta, 1, RED_LANES, st, P, P.part);
             if (P.refOrder) launch_pdl(k_update_s<false>, nblk(maxRows), TB, st, P, s, z);

@@ -52,7 +52,8 @@ constexpr int REF_MAX_WORKERS = 256;  // worker count of the reference-order mea
 
 // scalars of the PCG kept on the device
 enum { SC_RESID0 = 0, SC_TOL, SC_RHO, SC_RESID, SC_ALPHA, SC_BETA, SC_COUNT };
-enum { ISC_ITERS = 0, ISC_CONVERGED, ISC_COUNT };
+// ISC_TICKETS: three counters of finished blocks (last_block, astg_pcg.cu), 0 between kernels
+enum { ISC_ITERS = 0, ISC_CONVERGED, ISC_TICKETS, ISC_COUNT = ISC_TICKETS + 3 };
 
 // Projection workspace (device pointers unless noted); sized for S + H rows.
 struct Proj {
@@ -66,7 +67,8 @@ struct Proj {
     int* pT;       // S
     int* rowCnt;   // rows
     int* rowPtr;   // rows + 1
-    int* padCol;   // rows * ROW_W
+    int* padCol;   // rows * ROW_W; after the assembly, with padVal: the first entries of the rows in quads
+                   // (k_row_quads)
     double* padVal;
     double* bRaw;  // rows
     int* col;      // rows * ROW_W (CSR, compacted)
@@ -110,6 +112,7 @@ struct Proj {
     // padded level-ordered records of the level-barrier fused preconditioner (entry e of row p at
     // e * rowsCap + p)
     int rowsCap;
+    int rows;      // the current system's, from the host (select_preconditioner): sizes the launches
     int* pos;        // rows: level position of each row (inverse of perm)
     int* lcntF;      // rows: lower entries of the row at level position p
     int* lcntB;
@@ -146,7 +149,7 @@ struct Proj {
     // mixed precision: FP32 copy of the matrix, FP32 inner vectors
     int pcActive32;   // the current solve can run the FP32 barrier-free preconditioner
     size_t pcSmem32;  // its dynamic shared memory per CTA
-    float* val32;     // rowsCap * ROW_W
+    float* val32;     // the rows' first entries in quads, rowsCap * 8
     float* e32;       // inner correction
     float* r32;       // inner residual
     float* s32;

@@ -203,15 +203,35 @@ static void launch_pdl(void (*k)(KArgs...), int grid, int block, cudaStream_t st
 }
 
 // ------------------------------------------------------------------ fixed-tree reduction
-__device__ inline double block_tree(double v, double* sh) {
-    int t = threadIdx.x;
-    sh[t] = v;
+// The sum of the RED_LANES lanes' values by halving (lane t adds lane t + 128, then t + 64, ... t + 1):
+// warp 0 folds eight values per lane, then by shuffles.  One barrier on each side; the tree over the
+// whole block had eight, and its lanes past the half issued their predicated-off FP64 additions at
+// full cost (~17 cycles a warp: 4 us of an SpMV block's 32 warps).  Every thread of the block calls it
+// (threads past RED_LANES with no value) and gets the sum.
+__device__ __forceinline__ double warp_tree(const double* sh) {  // one warp; the sum in lane 0
+    const int t = threadIdx.x & 31;
+    double a[RED_LANES / 32];
+#pragma unroll
+    for (int k = 0; k < RED_LANES / 32; ++k) a[k] = sh[t + 32 * k];
+#pragma unroll
+    for (int st = RED_LANES / 64; st >= 1; st >>= 1)
+#pragma unroll
+        for (int k = 0; k < st; ++k) a[k] = a[k] + a[k + st];
+    double s = a[0];
+#pragma unroll
+    for (int st = 16; st >= 1; st >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, st);
+    return s;
+}
+__device__ __forceinline__ double block_tree(double v, double* sh) {
+    const int t = threadIdx.x;
+    if (t < RED_LANES) sh[t] = v;
     __syncthreads();
-    for (int st = RED_LANES / 2; st >= 1; st >>= 1) {
-        if (t < st) sh[t] = sh[t] + sh[t + st];
-        __syncthreads();
+    if (t < 32) {
+        const double s = warp_tree(sh);
+        if (t == 0) sh[0] = s;
     }
-    double r = sh[0];
+    __syncthreads();
+    const double r = sh[0];
     __syncthreads();
     return r;
 }
@@ -229,29 +249,29 @@ __global__ void k_tree_sum(const double* a, const long long* nptr, long long nco
     double r = block_tree(acc, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
-// sum of a[i] * b[i]; each lane accumulates with fused multiply-adds (the library's order)
-__global__ void k_tree_dot(const double* a, const double* b, const int* nptr, double* part) {
-    grid_dep_wait();
-    __shared__ double sh[RED_LANES];
-    long long n = *nptr;
-    long long base = (long long)blockIdx.x * RED_CHUNK;
-    if (base >= n && blockIdx.x > 0) return;
-    double acc = 0.0;
-    for (int k = 0; k < RED_PER_LANE; ++k) {
-        long long i = base + threadIdx.x + (long long)RED_LANES * k;
-        if (i < n) acc = fma(a[i], b[i], acc);
-    }
-    double r = block_tree(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
-}
 // one block: folds m <= 2048 chunk partials with the same rule
 __device__ inline double fold_partials(const double* part, long long m, double* sh) {
     double acc = 0.0;
     for (int k = 0; k < RED_PER_LANE; ++k) {
         long long i = threadIdx.x + (long long)RED_LANES * k;
-        if (i < m) acc = acc + part[i];
+        if (i < m) acc = acc + __ldcg(part + i);
     }
     return block_tree(acc, sh);
+}
+
+// Counts the kernel's finished blocks; true in the last of `blocks`, which sees what the others had
+// written (by the thread that counts, 0) and leaves the counter at 0.  What follows a reduction in an
+// iteration -- alpha, beta, the stopping test -- is a few hundred cycles of one block: in the
+// reduction's last block it costs about 2 us, as a kernel of its own 3.5 to 5.
+__device__ __forceinline__ bool last_block(int* ticket, int blocks) {
+    __shared__ int last;
+    if (threadIdx.x == 0) {
+        unsigned k;
+        asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(k) : "l"(ticket), "r"(blocks - 1) : "memory");
+        last = k == (unsigned)(blocks - 1);
+    }
+    __syncthreads();
+    return last != 0;
 }
 
 // ------------------------------------------------------------------ reference-order reductions
@@ -895,7 +915,7 @@ __global__ void k_zero_rows(Proj P, int maxRows) {
 }
 void launch_assemble(const Dev& d, const Fields& F, const uint8_t* open, Proj& P, const int* hoPtr, const int* hoIdx,
                      double dt, cudaStream_t st) {
-    int maxRows = P.rowsCap;
+    const int maxRows = P.rows;
     ASTG_LAUNCH(k_zero_rows<<<nblk(maxRows), TB, 0, st>>>(P, maxRows));
     ASTG_LAUNCH(k_asm_oct<<<nblk(d.S), TB, 0, st>>>(d, F, P, hoPtr, hoIdx));
     ASTG_LAUNCH(k_asm_tilt<<<nblk(d.S), TB, 0, st>>>(d, F, P, open));
@@ -1887,7 +1907,7 @@ __global__ void k_item_fill(Proj P, int dir) {
 // false when the items do not fit their arrays (a matrix of very many, very narrow levels): the
 // caller takes another form of the sweeps
 static bool launch_item_schedule(Proj& P, cudaStream_t st) {
-    const int maxRows = P.rowsCap;
+    const int maxRows = P.rows;
     cudaMemsetAsync(P.nLevels, 0, sizeof(int), st);
     ASTG_LAUNCH(k_seg_levels<<<std::min(nblk(maxRows), 512), TB, 0, st>>>(P));
     ASTG_LAUNCH(k_seg_clear<<<64, TB, 0, st>>>(P));
@@ -1911,7 +1931,7 @@ void launch_level_schedule(const Dev& d, Proj& P, bool owner, cudaStream_t st) {
         P.pcActive32 = 0;
         if (P.clusterSize <= 0) return;
     }
-    int maxRows = P.rowsCap;
+    const int maxRows = P.rows;
     ASTG_LAUNCH(k_level_reset<<<nblk(maxRows + 1), TB, 0, st>>>(P, maxRows));
     ASTG_LAUNCH(k_level_hist<<<nblk(maxRows), TB, 0, st>>>(P));
 
@@ -1989,30 +2009,6 @@ __global__ void k_to_wave_order(Proj P, const double* r) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *P.nDof) wave_put_r(P, i, r[i]);
 }
-// z . r in the fixed tree's order after the wavefront preconditioner, whose cells' result is in its
-// own order: brought into the system's on the way.  (Written by the sweep itself, a step's 32 rows
-// would be 32 separate sectors on the one warp that the sweep waits for: 100 cycles a step.)
-__global__ void k_tree_dot_wave(Proj P, double* z, const double* r, double* part) {
-    grid_dep_wait();
-    __shared__ double sh[RED_LANES];
-    if (*P.done) return;
-    const int n = *P.nDof, nx = P.wnx, nc = nx * P.wny;
-    const long long base = (long long)blockIdx.x * RED_CHUNK + threadIdx.x;
-    if (base - threadIdx.x >= n) return;
-    double acc = 0;
-#pragma unroll
-    for (int k = 0; k < RED_PER_LANE; ++k) {
-        const long long i = base + (long long)RED_LANES * k;
-        if (i < n) {
-            double zi;
-            if (i < nc) z[i] = zi = P.wZ[wave_slot((int)i % nx, (int)i / nx, P.wny)];
-            else zi = z[i];
-            acc = fma(zi, r[i], acc);
-        }
-    }
-    const double s = block_tree(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
 __global__ void k_zero_vec(double* a, const int* nptr) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *nptr) a[i] = 0;
@@ -2021,25 +2017,29 @@ __global__ void k_zero_vec(double* a, const int* nptr) {
 // the largest of the block's v (all threads of the block call it) into *out: a warp maximum by
 // shuffles, the block's over its warps in shared memory, one atomic per block (non-negative doubles
 // order as their bit patterns).  One atomic per warp on the same word serialised at the L2.
-__device__ __forceinline__ void block_absmax_to(double v, unsigned long long* out) {
-    __shared__ double wm[32];
+// The comparisons are the integers': the FP64 pipe is the slow one.  A NaN counts as 0.
+typedef unsigned long long AbsBits;
+__device__ __forceinline__ AbsBits abs_bits(double v) {
+    const AbsBits b = (AbsBits)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+    return b > 0x7FF0000000000000ull ? 0 : b;
+}
+__device__ __forceinline__ void block_absmax_to(AbsBits v, unsigned long long* out) {
+    __shared__ AbsBits wm[32];
     for (int o = 16; o > 0; o >>= 1) {
-        double w = __shfl_xor_sync(0xffffffffu, v, o);
+        const AbsBits w = __shfl_xor_sync(0xffffffffu, v, o);
         v = w > v ? w : v;
     }
     if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double m = wm[0];
+        AbsBits m = wm[0];
         for (int k = 1; k < (int)((blockDim.x + 31) >> 5); ++k) m = wm[k] > m ? wm[k] : m;
-        if (m > 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+        if (m > 0) atomicMax(out, m);
     }
 }
 __global__ void k_absmax(const double* a, const int* nptr, unsigned long long* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v = 0;
-    if (i < *nptr) v = fabs(a[i]);
-    block_absmax_to(v, out);
+    block_absmax_to(i < *nptr ? abs_bits(a[i]) : 0, out);
 }
 __global__ void k_pcg_start(Proj P, const double* partRho, double tolFactor) {
     __shared__ double sh[RED_LANES];
@@ -2058,21 +2058,25 @@ __global__ void k_pcg_start(Proj P, const double* partRho, double tolFactor) {
         *P.amax = 0;
     }
 }
-// z = A s, partial dots of s . z (lane layout of the fixed tree: thread t owns rows t + 256 k)
-// y = A s over one chunk of RED_CHUNK rows, SPMV_THREADS threads per chunk (each row summed in
-// column order by one thread, staged in shared memory), then the chunk's partial of s . y in the
-// fixed tree's order: lane t adds rows t, t + 256, ... of the chunk, the lanes fold by halving.
-// Four times the threads of one lane per 8 rows, same values bit for bit.
-constexpr int SPMV_THREADS = 1024;
-__device__ __forceinline__ double chunk_fold(double acc, double* sh) {
-    const int t = threadIdx.x;
-    if (t < RED_LANES) sh[t] = acc;
-    __syncthreads();
-    for (int st = RED_LANES / 2; st >= 1; st >>= 1) {
-        if (t < st) sh[t] = sh[t] + sh[t + st];
-        __syncthreads();
-    }
-    return sh[0];
+// y = A s and the partial dots s . y.  A chunk of RED_CHUNK rows takes a cluster of SPMV_CTAS CTAs, a
+// thread one row (summed in column order).  CTA j has the rows of the fixed tree's lanes 32 j ... (of
+// lane t: t, t + 256, ...), warp k their k-th rows, so a lane's sum stays in the CTA; the lanes' sums
+// meet in the first CTA, which folds them by halving.  The last chunk to finish folds the partials
+// into alpha.  Bound by latency (launch, loads, the chains of FP64 operations at ~67 cycles each, the
+// hand-overs) and, few rows to an SM, by its FP64 pipe.  As one CTA of 1024 threads per chunk 20.2 us at
+// 288 k rows and 15.3 us at 1.4 k (GB300, alpha included); now 14.5 and 6.7 us.
+constexpr int SPMV_CTAS = RED_LANES / 32;
+constexpr int SPMV_THREADS = RED_CHUNK / SPMV_CTAS;
+static_assert(SPMV_THREADS == 32 * RED_PER_LANE, "a warp per row of the lanes");
+// the last block of s . q's partials: their fold (fold_partials' order, on SPMV_THREADS threads), alpha
+__device__ __forceinline__ void fold_alpha(const Proj& P, const double* part, double rho, double* sh) {
+    const int m = (*P.nDof + RED_CHUNK - 1) / RED_CHUNK;
+    if (!last_block(P.isc + ISC_TICKETS + 1, m)) return;
+    double acc = 0.0;
+    if (threadIdx.x < RED_LANES)
+        for (int i = threadIdx.x; i < m; i += RED_LANES) acc = acc + __ldcg(part + i);
+    const double dsz = block_tree(acc, sh);
+    if (threadIdx.x == 0) P.sc[SC_ALPHA] = rho / dsz;
 }
 // FUSED (the library's order): each product-accumulate is one fused multiply-add; otherwise (the
 // reference's order) a product, then an addition, as its CSR multiply computes them
@@ -2082,36 +2086,129 @@ __device__ __forceinline__ double mac_add(double acc, double a, double b) {
     double prod = a * b;
     return acc + prod;
 }
-template <bool FUSED>
-__global__ void __launch_bounds__(SPMV_THREADS) k_spmv_dot(Proj P, const double* s, double* z, double* part) {
+// acc += v[e] x[e] (fused) for the first w of four entries, in order; this lane has `mine` of them.
+// w (of the warp) is a jump: a predicated-off FP64 instruction takes the pipe like one that runs.
+__device__ __forceinline__ double row_chain(double acc, int w, int mine, const double* v, const double* x) {
+    asm volatile(
+        "{.reg .pred p0, p1, p2, p3;\n\t"
+        "setp.gt.s32 p0, %2, 0; setp.gt.s32 p1, %2, 1; setp.gt.s32 p2, %2, 2; setp.gt.s32 p3, %2, 3;\n\t"
+        "ts_%=: .branchtargets L1_%=, L2_%=, L3_%=, L4_%=;\n\t"
+        "brx.idx.uni %1, ts_%=;\n\t"
+        "L4_%=: @p0 fma.rn.f64 %0, %3, %7, %0; @p1 fma.rn.f64 %0, %4, %8, %0;"
+        " @p2 fma.rn.f64 %0, %5, %9, %0; @p3 fma.rn.f64 %0, %6, %10, %0; bra.uni E_%=;\n\t"
+        "L3_%=: @p0 fma.rn.f64 %0, %3, %7, %0; @p1 fma.rn.f64 %0, %4, %8, %0; @p2 fma.rn.f64 %0, %5, %9, %0; bra.uni E_%=;\n\t"
+        "L2_%=: @p0 fma.rn.f64 %0, %3, %7, %0; @p1 fma.rn.f64 %0, %4, %8, %0; bra.uni E_%=;\n\t"
+        "L1_%=: @p0 fma.rn.f64 %0, %3, %7, %0;\n\t"
+        "E_%=:}"
+        : "+d"(acc)
+        : "r"(w - 1), "r"(mine), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]), "d"(x[0]), "d"(x[1]), "d"(x[2]), "d"(x[3]));
+    return acc;
+}
+__device__ __forceinline__ float row_chain(float acc, int, int mine, const float* v, const float* x) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        if (e < mine) acc = fmaf(v[e], x[e], acc);
+    return acc;
+}
+// The first eight entries of every row, entry quads by rows: columns at padCol, values at padVal (and
+// val32), arrays of the assembly that are free once the CSR form stands.  A warp's 32 rows then read
+// 4 lines per 16 bytes a lane; row by row from the CSR arrays each entry was 21 lines, and the columns
+// came a latency behind the row pointers: SpMV + dot at 288 k rows 17.2 -> 16.5 us, at 1.4 k 8.4 -> 7.9.
+__global__ void k_row_quads(Proj P, bool fp32) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= *P.nDof) return;
+    const int q0 = P.rowPtr[r], q1 = P.rowPtr[r + 1];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        int c[4];
+        double v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int q = q0 + 4 * u + e;
+            c[e] = q < q1 ? P.col[q] : 0;
+            v[e] = q < q1 ? P.val[q] : 0.0;
+        }
+        const size_t at = (size_t)u * P.rows + r;
+        reinterpret_cast<int4*>(P.padCol)[at] = make_int4(c[0], c[1], c[2], c[3]);
+        reinterpret_cast<double2*>(P.padVal)[2 * (size_t)u * P.rows + r] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2*>(P.padVal)[(2 * (size_t)u + 1) * P.rows + r] = make_double2(v[2], v[3]);
+        if (fp32) reinterpret_cast<float4*>(P.val32)[at] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+    }
+}
+__device__ __forceinline__ void quad_vals(const Proj& P, int u, int row, double* v) {
+    const double2 a = reinterpret_cast<const double2*>(P.padVal)[2 * (size_t)u * P.rows + row];
+    const double2 b = reinterpret_cast<const double2*>(P.padVal)[(2 * (size_t)u + 1) * P.rows + row];
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+__device__ __forceinline__ void quad_vals(const Proj& P, int u, int row, float* v) {
+    const float4 a = reinterpret_cast<const float4*>(P.val32)[(size_t)u * P.rows + row];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+}
+// One row of A s per lane, entries in column order, fused; all lanes of the warp call it (row < 0: 0).
+template <typename T>
+__device__ __forceinline__ T row_product(const Proj& P, const T* s, int row) {
+    const int r = max(row, 0), q0 = P.rowPtr[r], len = row >= 0 ? P.rowPtr[r + 1] - q0 : 0;
+    T v[8], x[8], t = 0;
+    const int4 c0 = reinterpret_cast<const int4*>(P.padCol)[r], c1 = reinterpret_cast<const int4*>(P.padCol)[(size_t)P.rows + r];
+    quad_vals(P, 0, r, v);
+    quad_vals(P, 1, r, v + 4);
+    const int c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = s[c[e]];
+    const int most = __reduce_max_sync(0xffffffffu, len);
+    if (most > 0) t = row_chain(t, min(4, most), len, v, x);
+    if (most > 4) t = row_chain(t, min(4, most - 4), len - 4, v + 4, x + 4);
+    for (int b = 8; b < most; b += 4) {  // rows at level changes
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int q = min(q0 + b + e, q0 + max(len - 1, 0));
+            v[e] = (T)P.val[q];
+            x[e] = s[P.col[q]];
+        }
+        t = row_chain(t, min(4, most - b), len - b, v, x);
+    }
+    return t;
+}
+template <typename T, bool FUSED>
+__global__ void __cluster_dims__(SPMV_CTAS, 1, 1) __launch_bounds__(SPMV_THREADS, 4)
+    k_spmv_dot(Proj P, const T* s, T* y, double* part) {
     grid_dep_wait();
-    __shared__ double ys[RED_CHUNK];
+    __shared__ T ss[SPMV_THREADS], ys[SPMV_THREADS];
     __shared__ double sh[RED_LANES];
     if (*P.done) return;
-    int n = *P.nDof;
-    long long base = (long long)blockIdx.x * RED_CHUNK;
+    const int n = *P.nDof, chunk = blockIdx.x / SPMV_CTAS, rank = blockIdx.x % SPMV_CTAS;
+    const long long base = (long long)chunk * RED_CHUNK;
     if (base >= n) return;
-    for (int k = threadIdx.x; k < RED_CHUNK; k += SPMV_THREADS) {
-        long long i = base + k;
-        double t = 0;
-        if (i < n) {
-            for (int q = P.rowPtr[i]; q < P.rowPtr[i + 1]; ++q) t = mac_add<FUSED>(t, P.val[q], s[P.col[q]]);
-            z[i] = t;
-        }
-        ys[k] = t;
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // this CTA runs
+    const double rho = P.sc[SC_RHO];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long i = base + RED_LANES * warp + 32 * rank + lane;
+    T t = 0;
+    if (FUSED) t = row_product(P, s, i < n ? (int)i : -1);
+    else if (i < n)
+        for (int q = P.rowPtr[i]; q < P.rowPtr[i + 1]; ++q) t = mac_add<false>(t, (T)P.val[q], s[P.col[q]]);
+    if (i < n) {
+        y[i] = t;
+        ss[threadIdx.x] = s[i];
+        ys[threadIdx.x] = t;
     }
     __syncthreads();
-    const int tl = threadIdx.x;
-    double acc = 0.0;
-    if (tl < RED_LANES)
-        for (int k = 0; k < RED_PER_LANE; ++k) {
-            long long i = base + tl + (long long)RED_LANES * k;
-            if (i < n) acc = mac_add<FUSED>(acc, s[i], ys[tl + RED_LANES * k]);
-        }
-    double r = chunk_fold(acc, sh);
-    if (tl == 0) part[blockIdx.x] = r;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 0) {
+        double acc = 0.0;
+        for (int k = 0; k < RED_PER_LANE && i + RED_LANES * k < n; ++k) acc = mac_add<FUSED>(acc, (double)ss[lane + 32 * k], (double)ys[lane + 32 * k]);
+        *cg::this_cluster().map_shared_rank(sh + 32 * rank + lane, 0) = acc;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (rank != 0) return;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 0) {
+        const double r = warp_tree(sh);
+        if (lane == 0) part[chunk] = r;
+    }
+    if (FUSED) fold_alpha(P, part, rho, sh);  // the reference's order folds its own way first
 }
-__global__ void k_alpha(Proj P, const double* part) {
+__global__ void k_alpha(Proj P, const double* part) {  // reference order only
     grid_dep_wait();
     __shared__ double sh[RED_LANES];
     if (*P.done) return;
@@ -2120,54 +2217,83 @@ __global__ void k_alpha(Proj P, const double* part) {
     double dsz = fold_partials(part, m, sh);
     if (threadIdx.x == 0) P.sc[SC_ALPHA] = P.sc[SC_RHO] / dsz;
 }
+// the stopping test, by one thread after every block's |r|
+__device__ __forceinline__ void check_residual(const Proj& P, int maxIter) {
+    const double res = __longlong_as_double((long long)__ldcg(P.amax));
+    *P.amax = 0;
+    const int it = P.isc[ISC_ITERS] + 1;
+    P.sc[SC_RESID] = res;
+    P.isc[ISC_ITERS] = it;
+    if (res <= P.sc[SC_TOL]) {
+        P.isc[ISC_CONVERGED] = 1;
+        *P.done = 1;
+    } else if (it >= maxIter) {
+        P.isc[ISC_CONVERGED] = 0;
+        *P.done = 1;
+    }
+}
 template <bool FUSED>
-__global__ void k_update_xr(Proj P, double* x, double* r, const double* s, const double* z) {
+__global__ void k_update_xr(Proj P, double* x, double* r, const double* s, const double* z, int maxIter) {
     grid_dep_wait();
     if (*P.done) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int n = *P.nDof;
-    double alpha = P.sc[SC_ALPHA];
-    double v = 0;
-    if (i < n) {
+    const int n = *P.nDof;
+    const double alpha = P.sc[SC_ALPHA];
+    AbsBits v = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         x[i] = mac_add<FUSED>(x[i], alpha, s[i]);
         double ri = mac_add<FUSED>(r[i], -alpha, z[i]);
         r[i] = ri;
         if (P.rl && P.pcActive) P.rl[P.pos[i]] = ri;  // level-barrier form
         if (P.wave) wave_put_r(P, i, ri);
-        v = fabs(ri);
+        const AbsBits a = abs_bits(ri);
+        v = a > v ? a : v;
     }
     block_absmax_to(v, P.amax);
+    if (last_block(P.isc + ISC_TICKETS + 2, gridDim.x) && threadIdx.x == 0) check_residual(P, maxIter);
 }
-__global__ void k_check(Proj P, int maxIter) {
-    grid_dep_wait();
-    if (*P.done) return;
-    double res = __longlong_as_double((long long)*P.amax);
-    *P.amax = 0;
-    int it = P.isc[ISC_ITERS];
-    P.sc[SC_RESID] = res;
-    if (res <= P.sc[SC_TOL]) {
-        P.isc[ISC_ITERS] = it + 1;
-        P.isc[ISC_CONVERGED] = 1;
-        *P.done = 1;
-    } else if (it + 1 >= maxIter) {
-        P.isc[ISC_ITERS] = it + 1;
-        P.isc[ISC_CONVERGED] = 0;
-        *P.done = 1;
-    } else {
-        P.isc[ISC_ITERS] = it + 1;
-    }
+__device__ __forceinline__ void set_beta(const Proj& P, double rn, double rho) {
+    P.sc[SC_BETA] = rn / rho;
+    P.sc[SC_RHO] = rn;
 }
-__global__ void k_beta(Proj P, const double* part) {
+__global__ void k_beta(Proj P, const double* part) {  // reference order only
     grid_dep_wait();
     __shared__ double sh[RED_LANES];
     if (*P.done) return;
     int n = *P.nDof;
     long long m = (n + RED_CHUNK - 1) / RED_CHUNK;
     double rn = fold_partials(part, m, sh);
-    if (threadIdx.x == 0) {
-        P.sc[SC_BETA] = rn / P.sc[SC_RHO];
-        P.sc[SC_RHO] = rn;
+    if (threadIdx.x == 0) set_beta(P, rn, P.sc[SC_RHO]);
+}
+// z . r in the fixed tree's order, each lane accumulating with fused multiply-adds; BETA: then the
+// iteration's beta.  WAVE: the cells' z is in the wavefront preconditioner's order and is brought into
+// the system's on the way (written by the sweep itself it would cost that one warp's time).
+template <typename T, bool WAVE, bool BETA>
+__global__ void k_dot_zr(Proj P, T* z, const T* r, double* part) {
+    grid_dep_wait();
+    __shared__ double sh[RED_LANES];
+    if (*P.done) return;
+    const int n = *P.nDof, nx = P.wnx, nc = nx * P.wny;
+    const long long base = (long long)blockIdx.x * RED_CHUNK;
+    if (base >= n) return;
+    const double rho = BETA ? P.sc[SC_RHO] : 0;
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < RED_PER_LANE; ++k) {
+        const long long i = base + threadIdx.x + (long long)RED_LANES * k;
+        if (i < n) {
+            T zi;
+            if (WAVE && i < nc) z[i] = zi = (T)P.wZ[wave_slot((int)i % nx, (int)i / nx, P.wny)];
+            else zi = z[i];
+            acc = fma((double)zi, (double)r[i], acc);
+        }
     }
+    const double s = block_tree(acc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    if (!BETA) return;
+    const int m = (n + RED_CHUNK - 1) / RED_CHUNK;
+    if (!last_block(P.isc + ISC_TICKETS, m)) return;
+    const double rn = fold_partials(part, m, sh);
+    if (threadIdx.x == 0) set_beta(P, rn, rho);
 }
 template <bool FUSED>
 __global__ void k_update_s(Proj P, double* s, const double* z) {
@@ -2181,6 +2307,7 @@ __global__ void k_reset_counter(int* c) { *c = 0; }
 
 // one preconditioner application z = (L L^T)^-1 r
 void select_preconditioner(Proj& P, int n) {
+    P.rows = std::max(n, 1);
     P.pcActive = 0;
     P.pcSmem = 0;
     P.pcActive32 = 0;
@@ -2374,8 +2501,9 @@ __global__ void k_mic_factor_plan(Dev d, Proj P, double omega, double minDiag, i
     }
 }
 void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epoch, cudaStream_t st, KProf* prof) {
-    int maxRows = P.rowsCap;
+    const int maxRows = P.rows;
     ASTG_LAUNCH(k_mic_init<<<nblk(maxRows), TB, 0, st>>>(P));
+    ASTG_LAUNCH(k_row_quads<<<nblk(maxRows), TB, 0, st>>>(P, P.val32 && P.pcActive32));
     ASTG_LAUNCH(k_reset_counter<<<1, 1, 0, st>>>(P.counter));
     bool plan = P.plan != nullptr;
     if (plan) {
@@ -2397,16 +2525,22 @@ void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epo
     prof_end(prof, st);
 }
 
+// Blocks of k_update_xr / k_update_er32: eight of TB threads per SM at most, each over several rows.  One
+// atomic on the same word per TB rows, half the blocks past the last row and FP64 comparisons made the
+// update 13 us at 288 k rows, the stopping test another 3.5; together now 7 us.
+static int update_blocks(int maxRows) { return std::min(nblk(maxRows), 152 * 8); }
+
 // Runs the FP64 PCG to completion.  Iterations are launched in batches; every kernel returns at
 // once when the device "done" flag is set, so a batch that overshoots does no work.
 int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& epoch, int batch, cudaStream_t st,
                     KProf* prof) {
-    int maxRows = P.rowsCap;
+    const int maxRows = P.rows;
     int chunks = (maxRows + RED_CHUNK - 1) / RED_CHUNK;
     double* x = P.x;
     double* r = P.r;
     double* s = P.s;
     double* z = P.z;
+    const int rowBlocks = update_blocks(maxRows);
     ASTG_LAUNCH(k_zero_vec<<<nblk(maxRows), TB, 0, st>>>(x, P.nDof));
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(P.b, r, P.nDof));
     cudaMemsetAsync(P.amax, 0, sizeof(unsigned long long), st);
@@ -2416,8 +2550,8 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
     if (P.wave) ASTG_LAUNCH(k_to_wave_order<<<nblk(maxRows), TB, 0, st>>>(P, r));
     precond(d, P, r, z, epoch, st, prof);
     if (P.refOrder) launch_dot_ref(z, r, P.nDof, P.part, st);
-    else if (P.wave) ASTG_LAUNCH(k_tree_dot_wave<<<chunks, RED_LANES, 0, st>>>(P, z, r, P.part));
-    else ASTG_LAUNCH(k_tree_dot<<<chunks, RED_LANES, 0, st>>>(z, r, P.nDof, P.part));
+    else if (P.wave) launch_pdl(k_dot_zr<double, true, false>, chunks, RED_LANES, st, P, z, r, P.part);
+    else launch_pdl(k_dot_zr<double, false, false>, chunks, RED_LANES, st, P, z, r, P.part);
     ASTG_LAUNCH(k_pcg_start<<<1, RED_LANES, 0, st>>>(P, P.part, tolFactor));
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(z, s, P.nDof));
     int launched = 0;
@@ -2425,25 +2559,30 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
     auto body = [&](int nb, KProf* pf) {
         for (int it = 0; it < nb; ++it) {
             prof_begin(pf, 2, st);
-            if (P.refOrder) launch_pdl(k_spmv_dot<false>, chunks, SPMV_THREADS, st, P, s, z, P.part);
-            else launch_pdl(k_spmv_dot<true>, chunks, SPMV_THREADS, st, P, s, z, P.part);
+            if (P.refOrder) launch_pdl(k_spmv_dot<double, false>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, z, P.part);
+            else launch_pdl(k_spmv_dot<double, true>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, z, P.part);
             prof_end(pf, st);
-            if (P.refOrder) launch_dot_ref(s, z, P.nDof, P.part, st);
-            launch_pdl(k_alpha, 1, RED_LANES, st, P, P.part);
-            if (P.refOrder) launch_pdl(k_update_xr<false>, nblk(maxRows), TB, st, P, x, r, s, z);
-            else launch_pdl(k_update_xr<true>, nblk(maxRows), TB, st, P, x, r, s, z);
-            launch_pdl(k_check, 1, 1, st, P, maxIter);
+            if (P.refOrder) {
+                launch_dot_ref(s, z, P.nDof, P.part, st);
+                launch_pdl(k_alpha, 1, RED_LANES, st, P, P.part);
+                launch_pdl(k_update_xr<false>, rowBlocks, TB, st, P, x, r, s, z, maxIter);
+            } else {
+                launch_pdl(k_update_xr<true>, rowBlocks, TB, st, P, x, r, s, z, maxIter);
+            }
             precond(d, P, r, z, epoch, st, pf);
-            if (P.refOrder) launch_dot_ref(z, r, P.nDof, P.part, st);
-            else if (P.wave) launch_pdl(k_tree_dot_wave, chunks, RED_LANES, st, P, z, r, P.part);
-            else launch_pdl(k_tree_dot, chunks, RED_LANES, st, z, r, P.nDof, P.part);
-            launch_pdl(k_beta, 1, RED_LANES, st, P, P.part);
-            if (P.refOrder) launch_pdl(k_update_s<false>, nblk(maxRows), TB, st, P, s, z);
-            else launch_pdl(k_update_s<true>, nblk(maxRows), TB, st, P, s, z);
+            if (P.refOrder) {
+                launch_dot_ref(z, r, P.nDof, P.part, st);
+                launch_pdl(k_beta, 1, RED_LANES, st, P, P.part);
+                launch_pdl(k_update_s<false>, nblk(maxRows), TB, st, P, s, z);
+            } else {
+                if (P.wave) launch_pdl(k_dot_zr<double, true, true>, chunks, RED_LANES, st, P, z, r, P.part);
+                else launch_pdl(k_dot_zr<double, false, true>, chunks, RED_LANES, st, P, z, r, P.part);
+                launch_pdl(k_update_s<true>, nblk(maxRows), TB, st, P, s, z);
+            }
         }
     };
     BatchGraph graph;
-    const bool graphs = g_pcg_graphs && (P.pcActive || P.clusterSize > 0);
+    const bool graphs = g_pcg_graphs && (P.wave || P.pcActive || P.clusterSize > 0);
     while (launched < maxIter) {
         int nb = batch;
         if (launched + nb > maxIter) nb = maxIter - launched;
@@ -2472,20 +2611,16 @@ namespace astg {
 // (fmaf / fma written out: the library is compiled without contraction for the FP64 paths).
 constexpr double MIXED_INNER_REDUCTION = 1e-5;
 constexpr int MIXED_MAX_OUTER = 20;
-__global__ void k_to_f32(const double* a, float* b, const int* nptr) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < *nptr) b[i] = (float)a[i];
-}
 // r = b - A x (FP64, row sums in column order), |r|_inf into amax
 __global__ void k_resid64(Proj P, const double* x, double* r) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v = 0;
+    AbsBits v = 0;
     if (i < *P.nDof) {
         double t = 0;
         for (int q = P.rowPtr[i]; q < P.rowPtr[i + 1]; ++q) t += P.val[q] * x[P.col[q]];
         double ri = P.b[i] - t;
         r[i] = ri;
-        v = fabs(ri);
+        v = abs_bits(ri);
     }
     block_absmax_to(v, P.amax);
 }
@@ -2496,20 +2631,6 @@ __global__ void k_inner_init(Proj P, const double* r) {
     float ri = (float)r[i];
     P.r32[i] = ri;
     P.e32[i] = 0.0f;
-}
-// partial dots of FP32 vectors, products and sums in FP64 (fixed tree)
-__global__ void k_tree_dot32(const float* a, const float* b, const int* nptr, double* part) {
-    __shared__ double sh[RED_LANES];
-    long long n = *nptr;
-    long long base = (long long)blockIdx.x * RED_CHUNK;
-    if (base >= n && blockIdx.x > 0) return;
-    double acc = 0.0;
-    for (int k = 0; k < RED_PER_LANE; ++k) {
-        long long i = base + threadIdx.x + (long long)RED_LANES * k;
-        if (i < n) acc = fma((double)a[i], (double)b[i], acc);
-    }
-    double r = block_tree(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
 // inner start: rho = z.r, tolerance of this inner solve; the iteration count carries on
 __global__ void k_inner_start(Proj P, const double* partRho, double innerTol) {
@@ -2528,48 +2649,24 @@ __global__ void k_copy32(const float* a, float* b, const int* nptr) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *nptr) b[i] = a[i];
 }
-// q = A32 s (FP32 row sums), partial dots s.q in FP64
-__global__ void __launch_bounds__(SPMV_THREADS) k_spmv32_dot(Proj P, const float* s, float* q, double* part) {
-    __shared__ float ys[RED_CHUNK];
-    __shared__ double sh[RED_LANES];
+__global__ void k_update_er32(Proj P, int maxIter) {
+    grid_dep_wait();
     if (*P.done) return;
-    int n = *P.nDof;
-    long long base = (long long)blockIdx.x * RED_CHUNK;
-    if (base >= n) return;
-    for (int k = threadIdx.x; k < RED_CHUNK; k += SPMV_THREADS) {
-        long long i = base + k;
-        float t = 0;
-        if (i < n) {
-            for (int c = P.rowPtr[i]; c < P.rowPtr[i + 1]; ++c) t = fmaf(P.val32[c], s[P.col[c]], t);
-            q[i] = t;
-        }
-        ys[k] = t;
-    }
-    __syncthreads();
-    const int tl = threadIdx.x;
-    double acc = 0.0;
-    if (tl < RED_LANES)
-        for (int k = 0; k < RED_PER_LANE; ++k) {
-            long long i = base + tl + (long long)RED_LANES * k;
-            if (i < n) acc = fma((double)s[i], (double)ys[tl + RED_LANES * k], acc);
-        }
-    double r = chunk_fold(acc, sh);
-    if (tl == 0) part[blockIdx.x] = r;
-}
-__global__ void k_update_er32(Proj P) {
-    if (*P.done) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float alpha = (float)P.sc[SC_ALPHA];
-    double v = 0;
-    if (i < *P.nDof) {
+    const int n = *P.nDof;
+    const float alpha = (float)P.sc[SC_ALPHA];
+    float v = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         P.e32[i] = fmaf(alpha, P.s32[i], P.e32[i]);
         float ri = fmaf(-alpha, P.q32[i], P.r32[i]);
         P.r32[i] = ri;
-        v = fabs((double)ri);
+        const float a = fabsf(ri);
+        v = a > v ? a : v;
     }
-    block_absmax_to(v, P.amax);
+    block_absmax_to(abs_bits((double)v), P.amax);
+    if (last_block(P.isc + ISC_TICKETS + 2, gridDim.x) && threadIdx.x == 0) check_residual(P, maxIter);
 }
 __global__ void k_update_s32(Proj P) {
+    grid_dep_wait();
     if (*P.done) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < *P.nDof) P.s32[i] = fmaf((float)P.sc[SC_BETA], P.s32[i], P.z32[i]);
@@ -2603,11 +2700,11 @@ static double read_amax(Proj& P, cudaStream_t st) {
 }
 int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int batch, cudaStream_t st, KProf* prof) {
     if (!P.pcActive32) return -1;
-    int maxRows = P.rowsCap;
+    const int maxRows = P.rows;
     int chunks = (maxRows + RED_CHUNK - 1) / RED_CHUNK;
     double* x = P.x;
     double* r = P.r;
-    ASTG_LAUNCH(k_to_f32<<<nblk((long long)maxRows * ROW_W), TB, 0, st>>>(P.val, P.val32, P.nnz));
+    const int rowBlocks = update_blocks(maxRows);
     ASTG_LAUNCH(k_zero_vec<<<nblk(maxRows), TB, 0, st>>>(x, P.nDof));
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(P.b, r, P.nDof));
     cudaMemsetAsync(P.amax, 0, sizeof(unsigned long long), st);
@@ -2635,24 +2732,21 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
         cudaError_t e = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
         prof_end(prof, st);
         if (e != cudaSuccess) g_cluster_error = e;
-        ASTG_LAUNCH(k_tree_dot32<<<chunks, RED_LANES, 0, st>>>(P.z32, P.r32, P.nDof, P.part));
+        launch_pdl(k_dot_zr<float, false, false>, chunks, RED_LANES, st, P, P.z32, P.r32, P.part);
         ASTG_LAUNCH(k_inner_start<<<1, RED_LANES, 0, st>>>(P, P.part, innerTol));
         ASTG_LAUNCH(k_copy32<<<nblk(maxRows), TB, 0, st>>>(P.z32, P.s32, P.nDof));
         auto body = [&](int nb, KProf* pf) {
             for (int it = 0; it < nb; ++it) {
                 prof_begin(pf, 2, st);
-                ASTG_LAUNCH(k_spmv32_dot<<<chunks, SPMV_THREADS, 0, st>>>(P, P.s32, P.q32, P.part));
+                launch_pdl(k_spmv_dot<float, true>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, P.s32, P.q32, P.part);
                 prof_end(pf, st);
-                ASTG_LAUNCH(k_alpha<<<1, RED_LANES, 0, st>>>(P, P.part));
-                ASTG_LAUNCH(k_update_er32<<<nblk(maxRows), TB, 0, st>>>(P));
-                ASTG_LAUNCH(k_check<<<1, 1, 0, st>>>(P, maxIter));
+                launch_pdl(k_update_er32, rowBlocks, TB, st, P, maxIter);
                 prof_begin(pf, 0, st);
                 cudaError_t pe = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
                 prof_end(pf, st);
                 if (pe != cudaSuccess) g_cluster_error = pe;
-                ASTG_LAUNCH(k_tree_dot32<<<chunks, RED_LANES, 0, st>>>(P.z32, P.r32, P.nDof, P.part));
-                ASTG_LAUNCH(k_beta<<<1, RED_LANES, 0, st>>>(P, P.part));
-                ASTG_LAUNCH(k_update_s32<<<nblk(maxRows), TB, 0, st>>>(P));
+                launch_pdl(k_dot_zr<float, false, true>, chunks, RED_LANES, st, P, P.z32, P.r32, P.part);
+                launch_pdl(k_update_s32, nblk(maxRows), TB, st, P);
             }
         };
         for (int launched = 0; launched < maxIter;) {
@@ -2772,7 +2866,7 @@ void proj_alloc(Proj& J, long long rows, int device, cudaStream_t st, std::vecto
         J.ownFill = A.get<int>((rows + 1) * J.pcCluster);
         J.itemPtr = A.get<int>((rows + 1) * J.pcCluster + 1);
         // FP32 copies for the mixed-precision solve
-        J.val32 = A.get<float>(rows * ROW_W);
+        J.val32 = A.get<float>(rows * 8);
         J.e32 = A.get<float>(rows);
         J.r32 = A.get<float>(rows);
         J.s32 = A.get<float>(rows);

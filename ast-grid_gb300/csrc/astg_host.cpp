@@ -955,6 +955,8 @@ struct astg_handle {
         ck(cudaMemcpyAsync(J.col, col, sizeof(int) * nnz, cudaMemcpyHostToDevice, st), "upload");
         ck(cudaMemcpyAsync(J.val, val, sizeof(double) * nnz, cudaMemcpyHostToDevice, st), "upload");
         select_preconditioner(J, n);
+        // more right-hand sides than such solves fit side by side: the form that shares SMs
+        if (J.pcAsync && nrhs > precond_concurrency(J, precision == ASTG_MIXED && J.pcActive32)) select_preconditioner(J, n, true);
         launch_external_system(d, J, n, st);
         checkStatus();
         bool mixed = precision == ASTG_MIXED && J.pcActive32;

@@ -283,7 +283,7 @@ int choose_cluster_size(int device);
 // cluster size (16 or 8) for the fused preconditioner (barrier-free form when async), or 0
 int choose_dsmem_cluster(bool async, size_t* smemMax);
 // per solve: whether the fused preconditioner holds a vector of n rows (sets pcActive, pcSmem)
-void select_preconditioner(Proj& P, int n);
+void select_preconditioner(Proj& P, int n, bool batch = false);
 extern cudaError_t g_cluster_error;  // last failed cluster launch (cudaSuccess if none)
 void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epoch, cudaStream_t st, KProf* prof);
 // the wavefront preconditioner z = (L L^T)^-1 r of a uniform 2-D system (Proj::wave), astg2d.cu

@@ -1291,7 +1291,7 @@ __global__ void __launch_bounds__(256, 1) k_precond_dsmem(Proj P, double* z, int
 // * The records bypass L1: at 150 KB of shared memory per CTA little L1 is left, and allocating
 //   there cost 7 % (238 -> 222 us).
 // * A scattered read of another CTA's slots takes ~3 cycles per lane, and 225 cycles at least, so
-//   rows are dealt in large blocks (select_preconditioner): 14 % of the entries cross CTAs instead of
+//   rows are dealt in large blocks (select_preconditioner): with three per CTA 14 % of the entries cross CTAs instead of
 //   34 % with blocks of 256 rows.
 constexpr long long PCA_SPIN_LIMIT = 1LL << 22;
 constexpr int PCA_MAX_WARPS = 16;
@@ -1565,7 +1565,8 @@ k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const in
     }
 }
 // how many clusters of the barrier-free preconditioner (FP64 or FP32 form) can be resident at
-// once, at most 8: the number of solves that can run side by side on disjoint SMs
+// once, at most 24: the number of solves that run side by side (20 right-hand sides at 42 k rows, 8
+// at a time 40 ms, 18 at a time 28 ms; a lane costs a host thread and ten vectors)
 int precond_concurrency(const Proj& P, bool fp32) {
     if (P.pcCluster <= 0) return 1;
     cudaLaunchConfig_t cfg = {};
@@ -1585,7 +1586,7 @@ int precond_concurrency(const Proj& P, bool fp32) {
         cudaGetLastError();
         nc = 1;
     }
-    return std::max(1, std::min(nc, 8));
+    return std::max(1, std::min(nc, 24));
 }
 static cudaError_t launch_precond_dsmem(const Proj& P, const double* r, double* z, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -2306,7 +2307,7 @@ __global__ void k_update_s(Proj P, double* s, const double* z) {
 __global__ void k_reset_counter(int* c) { *c = 0; }
 
 // one preconditioner application z = (L L^T)^-1 r
-void select_preconditioner(Proj& P, int n) {
+void select_preconditioner(Proj& P, int n, bool batch) {
     P.rows = std::max(n, 1);
     P.pcActive = 0;
     P.pcSmem = 0;
@@ -2320,10 +2321,14 @@ void select_preconditioner(Proj& P, int n) {
         P.pcSmem = bytes;
         return;
     }
-    const bool large = n > 100000;
-    P.pcWarps = large ? 12 : 8;
+    // us per PCG iteration on GB300, FP64 / FP32 form.  Warps per CTA: 22 k rows 8: 87 / 70, 12: 89 / 69;
+    // 42 k rows 8: 110 / 90, 12: 109 / 83; 305 k rows 12: 290 / 238, 16: 284 / 227.  Row blocks per CTA:
+    // 78 k rows 1: 142 / 114, 2: 146 / 112; 132 k rows 2: 181 / 141, 3: 193 / 156.  CTAs: 1.5 k rows
+    // one 46, eight 48 (FP64); 10.6 k rows 16 and 8 alike.  Many solves at once gain more from two
+    // CTAs to an SM, which 8 warps' registers allow (20 right-hand sides at 42 k rows 34 -> 28 ms).
+    P.pcWarps = batch ? 8 : n > 200000 ? 16 : n > 30000 ? 12 : 8;
     P.pcCS = n > 4096 ? P.pcCluster : 1;
-    const int blocks = large ? 3 : 1;
+    const int blocks = n > 100000 && !batch ? 2 : 1;
     P.pcBlock = (n + P.pcCS * blocks - 1) / (P.pcCS * blocks);
     P.pcChunk = P.pcBlock * blocks;
     const size_t slots = (size_t)P.pcChunk + 1;  // and the slot that holds 0

@@ -1635,6 +1635,7 @@ static PcaData<double> pca_data64(const Proj& P) {
     D.chunk = P.pcChunk;
     return D;
 }
+static void allow_mid_clusters();
 // Cluster size (16, else 8) at which the fused preconditioner (barrier-free form when async) can
 // run with the largest dynamic shared memory a CTA may have, or 0; *smemMax = that largest size.
 // Each solve then uses ceil(n / CS) doubles per CTA and falls back to the global-memory sweeps
@@ -1644,6 +1645,7 @@ int choose_dsmem_cluster(bool async, size_t* smemMax) {
     const int threads = async ? PCA_MAX_WARPS * 32 : PC_THREADS;
     *smemMax = 0;
     cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    allow_mid_clusters();
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -2146,7 +2148,8 @@ __device__ __forceinline__ void quad_vals(const Proj& P, int u, int row, float* 
     v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
 }
 // One row of A s per lane, entries in column order, fused; all lanes of the warp call it (row < 0: 0).
-template <typename T>
+// L2: s was written by other CTAs of the running kernel.
+template <typename T, bool L2 = false>
 __device__ __forceinline__ T row_product(const Proj& P, const T* s, int row) {
     const int r = max(row, 0), q0 = P.rowPtr[r], len = row >= 0 ? P.rowPtr[r + 1] - q0 : 0;
     T v[8], x[8], t = 0;
@@ -2155,7 +2158,7 @@ __device__ __forceinline__ T row_product(const Proj& P, const T* s, int row) {
     quad_vals(P, 1, r, v + 4);
     const int c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = s[c[e]];
+    for (int e = 0; e < 8; ++e) x[e] = L2 ? __ldcg(s + c[e]) : s[c[e]];
     const int most = __reduce_max_sync(0xffffffffu, len);
     if (most > 0) t = row_chain(t, min(4, most), len, v, x);
     if (most > 4) t = row_chain(t, min(4, most - 4), len - 4, v + 4, x + 4);
@@ -2164,7 +2167,7 @@ __device__ __forceinline__ T row_product(const Proj& P, const T* s, int row) {
         for (int e = 0; e < 4; ++e) {
             const int q = min(q0 + b + e, q0 + max(len - 1, 0));
             v[e] = (T)P.val[q];
-            x[e] = s[P.col[q]];
+            x[e] = L2 ? __ldcg(s + P.col[q]) : s[P.col[q]];
         }
         t = row_chain(t, min(4, most - b), len - b, v, x);
     }
@@ -2303,6 +2306,153 @@ __global__ void k_update_s(Proj P, double* s, const double* z) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= *P.nDof) return;
     s[i] = mac_add<FUSED>(z[i], P.sc[SC_BETA], s[i]);
+}
+// ------------------------------------------------------------------ one iteration's light work, small systems
+// What an iteration does between two applications of the preconditioner -- z . r, beta, s, A s, s . A s,
+// alpha, x, r, the stopping test -- as one cluster of 16 CTAs, for up to MID_MAX rows.  CTA j has lanes
+// 16 j ... of every chunk of the fixed tree (lane t: rows t, t + 256, ...), so each lane's sum is made in
+// one CTA; the lanes' sums go to every CTA, which folds them itself.  The same operations in the same
+// order as the kernels above.
+// Bound by latency: four grids, each a launch, the loads of flags, scalars and vectors and a fold whose
+// last block others wait for, against four cluster barriers (~0.2 us) and, towards MID_MAX, 16 SMs' FP64
+// pipes.  A whole iteration, FP64 / FP32, as four grids and as this one (GB300): 1.7 k rows 47 / 53 and
+// 37 / 42 us, 8 k rows 63 / 62 and 54 / 51, 15.6 k rows 77 / 70 and 72 / 62.
+constexpr int MID_CTAS = 16;
+constexpr int MID_THREADS = 512;
+constexpr int MID_CHUNKS = 8;
+constexpr int MID_MAX = MID_CHUNKS * RED_CHUNK;
+constexpr int MID_LANES = RED_LANES / MID_CTAS;           // tree lanes per CTA and chunk
+constexpr int MID_ROWS = MID_LANES * RED_PER_LANE;        // rows per CTA and chunk
+constexpr int MID_EACH = MID_CHUNKS * MID_ROWS / MID_THREADS;  // rows per thread
+static_assert(MID_ROWS % 32 == 0, "a chunk's rows of a CTA are whole warps");
+
+struct MidShared {
+    double lanes[MID_CHUNKS * RED_LANES];  // the lanes' sums, written by every CTA
+    double part[MID_CHUNKS];
+    double value;
+    AbsBits top[MID_CTAS];
+};
+// the fixed tree's sum of a . b over all rows, a and b staged by row slot (chunk, k, lane)
+template <typename T>
+__device__ __forceinline__ double mid_dot(cg::cluster_group& cl, MidShared& S, const T* a, const T* b, int n, int m) {
+    const int rank = cl.block_rank(), t = threadIdx.x;
+    __syncthreads();  // a and b staged
+    if (t < MID_LANES * m) {
+        const int c = t / MID_LANES, l = t % MID_LANES, row = c * RED_CHUNK + rank * MID_LANES + l;
+        double acc = 0.0;
+        for (int k = 0; k < RED_PER_LANE && row + RED_LANES * k < n; ++k)
+            acc = fma((double)a[c * MID_ROWS + k * MID_LANES + l], (double)b[c * MID_ROWS + k * MID_LANES + l], acc);
+        double* mine = S.lanes + c * RED_LANES + rank * MID_LANES + l;
+#pragma unroll
+        for (int q = 0; q < MID_CTAS; ++q) *cl.map_shared_rank(mine, q) = acc;
+    }
+    cl.sync();
+    if (t < 32 * m) {
+        const double s = warp_tree(S.lanes + (t >> 5) * RED_LANES);
+        if ((t & 31) == 0) S.part[t >> 5] = s;
+    }
+    __syncthreads();
+    double s = 0.0;
+    if (t < 32) {  // fold_partials with m <= 8 of its 256 lanes occupied: the others add 0
+        if (t < m) s = s + S.part[t];
+#pragma unroll
+        for (int st = MID_CHUNKS / 2; st >= 1; st >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, st);
+    }
+    return s;  // in thread 0
+}
+template <typename T, bool FIRST>
+__global__ void __cluster_dims__(MID_CTAS, 1, 1) __launch_bounds__(MID_THREADS, 1)
+    k_mid(Proj P, T* x, T* r, T* s, const T* z, int maxIter) {
+    __shared__ MidShared S;
+    __shared__ T sa[MID_CHUNKS * MID_ROWS], sb[MID_CHUNKS * MID_ROWS];
+    grid_dep_wait();
+    if (*P.done) return;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = cl.block_rank(), n = *P.nDof, m = (n + RED_CHUNK - 1) / RED_CHUNK, t = threadIdx.x;
+    const int nx = P.wnx, nc = P.wave ? nx * P.wny : 0;
+    double rho = P.sc[SC_RHO], beta = 0;
+    int row[MID_EACH];
+    T si[MID_EACH], ri[MID_EACH], yi[MID_EACH];
+#pragma unroll
+    for (int u = 0; u < MID_EACH; ++u) {
+        const int k = t + MID_THREADS * u, c = k / MID_ROWS, q = k % MID_ROWS;
+        const int i = c * RED_CHUNK + q / MID_LANES * RED_LANES + rank * MID_LANES + q % MID_LANES;
+        row[u] = c < m && i < n ? i : -1;
+        si[u] = ri[u] = 0;
+        if (row[u] >= 0) {
+            si[u] = s[i];
+            ri[u] = r[i];
+        }
+    }
+    cl.sync();  // every CTA runs
+    if (!FIRST) {
+        T zi[MID_EACH];
+#pragma unroll
+        for (int u = 0; u < MID_EACH; ++u) {
+            const int i = row[u];
+            zi[u] = 0;
+            if (i >= 0) zi[u] = i < nc ? (T)P.wZ[wave_slot(i % nx, i / nx, P.wny)] : z[i];
+            sa[t + MID_THREADS * u] = zi[u];
+            sb[t + MID_THREADS * u] = ri[u];
+        }
+        const double rn = mid_dot(cl, S, sa, sb, n, m);
+        if (t == 0) S.value = rn / rho;
+        __syncthreads();
+        beta = S.value;
+        if (t == 0) rho = rn;  // thread 0 alone goes on with it
+#pragma unroll
+        for (int u = 0; u < MID_EACH; ++u)
+            if (row[u] >= 0) {
+                si[u] = fma((T)beta, si[u], zi[u]);
+                __stcg(s + row[u], si[u]);
+            }
+        cl.sync();  // every row of s stands
+    }
+#pragma unroll
+    for (int u = 0; u < MID_EACH; ++u) {
+        if ((t & ~31) + MID_THREADS * u < MID_ROWS * m) yi[u] = row_product<T, true>(P, s, row[u]);
+        else yi[u] = 0;
+        sa[t + MID_THREADS * u] = si[u];
+        sb[t + MID_THREADS * u] = yi[u];
+    }
+    const double dsz = mid_dot(cl, S, sa, sb, n, m);
+    if (t == 0) S.value = rho / dsz;
+    __syncthreads();
+    const double alpha = S.value;
+    AbsBits top = 0;
+#pragma unroll
+    for (int u = 0; u < MID_EACH; ++u)
+        if (row[u] >= 0) {
+            const int i = row[u];
+            x[i] = fma((T)alpha, si[u], x[i]);
+            const T rv = fma(-(T)alpha, yi[u], ri[u]);
+            r[i] = rv;
+            if (P.wave && sizeof(T) == 8) wave_put_r(P, i, (double)rv);
+            const AbsBits a = abs_bits((double)rv);
+            top = a > top ? a : top;
+        }
+    __shared__ AbsBits wm[MID_THREADS / 32];
+    for (int o = 16; o > 0; o >>= 1) {
+        const AbsBits w = __shfl_xor_sync(0xffffffffu, top, o);
+        top = w > top ? w : top;
+    }
+    if ((t & 31) == 0) wm[t >> 5] = top;
+    __syncthreads();
+    if (t == 0) {
+        for (int k = 1; k < MID_THREADS / 32; ++k) top = wm[k] > top ? wm[k] : top;
+        *cl.map_shared_rank(&S.top[rank], 0) = top;
+    }
+    cl.sync();
+    if (rank == 0 && t == 0) {
+        for (int k = 1; k < MID_CTAS; ++k) top = S.top[k] > top ? S.top[k] : top;
+        *P.amax = top;
+        P.sc[SC_ALPHA] = alpha;
+        if (!FIRST) {
+            P.sc[SC_BETA] = beta;
+            P.sc[SC_RHO] = rho;
+        }
+        check_residual(P, maxIter);
+    }
 }
 __global__ void k_reset_counter(int* c) { *c = 0; }
 
@@ -2530,6 +2680,15 @@ void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epo
     prof_end(prof, st);
 }
 
+static void allow_mid_clusters() {
+    const void* k[4] = {(const void*)k_mid<double, true>, (const void*)k_mid<double, false>, (const void*)k_mid<float, true>,
+                        (const void*)k_mid<float, false>};
+    for (const void* f : k) cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+// The iteration's light work as k_mid: see there.  Profiling times the product by itself.
+static bool mid_fits(const Proj& P, const KProf* prof) {
+    return P.rows <= MID_MAX && P.pcCluster == MID_CTAS && !P.refOrder && !(prof && prof->on);
+}
 // Blocks of k_update_xr / k_update_er32: eight of TB threads per SM at most, each over several rows.  One
 // atomic on the same word per TB rows, half the blocks past the last row and FP64 comparisons made the
 // update 13 us at 288 k rows, the stopping test another 3.5; together now 7 us.
@@ -2561,8 +2720,18 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(z, s, P.nDof));
     int launched = 0;
     int hostDone = 0;
+    const bool mid = mid_fits(P, prof);
+    if (mid && maxIter > 0) {
+        launch_pdl(k_mid<double, true>, MID_CTAS, MID_THREADS, st, P, x, r, s, z, maxIter);
+        launched = 1;
+    }
     auto body = [&](int nb, KProf* pf) {
         for (int it = 0; it < nb; ++it) {
+            if (mid) {
+                precond(d, P, r, z, epoch, st, pf);
+                launch_pdl(k_mid<double, false>, MID_CTAS, MID_THREADS, st, P, x, r, s, z, maxIter);
+                continue;
+            }
             prof_begin(pf, 2, st);
             if (P.refOrder) launch_pdl(k_spmv_dot<double, false>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, z, P.part);
             else launch_pdl(k_spmv_dot<double, true>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, z, P.part);
@@ -2720,6 +2889,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
     double res = res0;
     int outer = 0, converged = 0;
     PcaData<float> D = pca_data32(P);
+    const bool mid = mid_fits(P, prof);
     BatchGraph graph;  // one inner batch; the same work in every outer cycle
     for (;;) {
         if (res <= tolAbs) {
@@ -2740,8 +2910,15 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
         launch_pdl(k_dot_zr<float, false, false>, chunks, RED_LANES, st, P, P.z32, P.r32, P.part);
         ASTG_LAUNCH(k_inner_start<<<1, RED_LANES, 0, st>>>(P, P.part, innerTol));
         ASTG_LAUNCH(k_copy32<<<nblk(maxRows), TB, 0, st>>>(P.z32, P.s32, P.nDof));
+        if (mid) launch_pdl(k_mid<float, true>, MID_CTAS, MID_THREADS, st, P, P.e32, P.r32, P.s32, P.z32, maxIter);
         auto body = [&](int nb, KProf* pf) {
             for (int it = 0; it < nb; ++it) {
+                if (mid) {
+                    cudaError_t pe = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
+                    if (pe != cudaSuccess) g_cluster_error = pe;
+                    launch_pdl(k_mid<float, false>, MID_CTAS, MID_THREADS, st, P, P.e32, P.r32, P.s32, (const float*)P.z32, maxIter);
+                    continue;
+                }
                 prof_begin(pf, 2, st);
                 launch_pdl(k_spmv_dot<float, true>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, P.s32, P.q32, P.part);
                 prof_end(pf, st);

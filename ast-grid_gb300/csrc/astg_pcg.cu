@@ -2579,7 +2579,11 @@ __global__ void k_plan_fill(Proj P) {
 }
 constexpr int PLAN_MAXU = 16;  // upper entries of a column applied from registers (more: in place)
 constexpr int FACTOR_ROW = 24;  // a row's upper entries updated in a thread-local copy (longer rows: in place)
-__global__ void k_mic_factor_plan(Dev d, Proj P, double omega, double minDiag, int epoch) {
+// lanes: rows per warp (the others of its threads leave).  Neighbouring rows depend on one another, and
+// a warp's diverged lanes run one after another: with 32 rows to a warp a level of the dependencies cost
+// ~12 us, with one ~6 -- as long as the warps' rows reach over enough of the grid.
+__global__ void k_mic_factor_plan(Dev d, Proj P, double omega, double minDiag, int epoch, int lanes) {
+    if ((int)(threadIdx.x & 31) >= lanes) return;
     int n = *P.nDof;
     for (;;) {
         int j = grab_row(P.counter);
@@ -2675,7 +2679,10 @@ void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epo
         if (plan) ASTG_LAUNCH(k_plan_fill<<<nblk(maxRows), TB, 0, st>>>(P));
     }
     prof_begin(prof, 3, st);
-    if (plan) ASTG_LAUNCH(k_mic_factor_plan<<<P.sweepBlocks, 128, 0, st>>>(d, P, omega, minDiag, ++epoch));
+    // us at 1 / 2 / 4 / 32 rows per warp (GB300): 10.5 k rows 352 / 406 / 446 / 614, 21 k 693 / 546 / 587 /
+    // 759, 40 k 1234 / 858 / 708 / 909, 125 k 4731 / 3091 / 2141 / 1171
+    const int lanes = maxRows <= 14000 ? 1 : maxRows <= 28000 ? 2 : maxRows <= 56000 ? 4 : 32;
+    if (plan) ASTG_LAUNCH(k_mic_factor_plan<<<P.sweepBlocks, 128, 0, st>>>(d, P, omega, minDiag, ++epoch, lanes));
     else ASTG_LAUNCH(k_mic_factor<<<P.sweepBlocks, 128, 0, st>>>(d, P, omega, minDiag, ++epoch));
     prof_end(prof, st);
 }

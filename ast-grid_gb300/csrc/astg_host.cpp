@@ -955,8 +955,13 @@ struct astg_handle {
         ck(cudaMemcpyAsync(J.col, col, sizeof(int) * nnz, cudaMemcpyHostToDevice, st), "upload");
         ck(cudaMemcpyAsync(J.val, val, sizeof(double) * nnz, cudaMemcpyHostToDevice, st), "upload");
         select_preconditioner(J, n);
-        // more right-hand sides than such solves fit side by side: the form that shares SMs
-        if (J.pcAsync && nrhs > precond_concurrency(J, precision == ASTG_MIXED && J.pcActive32)) select_preconditioner(J, n, true);
+        // more right-hand sides than such solves fit side by side: the form that shares SMs, if it does
+        if (J.pcAsync) {
+            const bool fp32 = precision == ASTG_MIXED && J.pcActive32;
+            const int alone = precond_concurrency(J, fp32);
+            if (nrhs > alone) select_preconditioner(J, n, true);
+            if (nrhs > alone && precond_concurrency(J, fp32) <= alone) select_preconditioner(J, n);
+        }
         launch_external_system(d, J, n, st);
         checkStatus();
         bool mixed = precision == ASTG_MIXED && J.pcActive32;

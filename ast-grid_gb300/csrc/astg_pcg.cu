@@ -2692,9 +2692,10 @@ static void allow_mid_clusters() {
                         (const void*)k_mid<float, false>};
     for (const void* f : k) cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
-// The iteration's light work as k_mid: see there.  Profiling times the product by itself.
+// The iteration's light work as k_mid: see there.  The level-barrier preconditioner wants the residual
+// in its own order (k_update_xr); profiling times the product by itself.
 static bool mid_fits(const Proj& P, const KProf* prof) {
-    return P.rows <= MID_MAX && P.pcCluster == MID_CTAS && !P.refOrder && !(prof && prof->on);
+    return P.rows <= MID_MAX && P.pcAsync && P.pcCluster == MID_CTAS && !P.refOrder && !(prof && prof->on);
 }
 // Blocks of k_update_xr / k_update_er32: eight of TB threads per SM at most, each over several rows.  One
 // atomic on the same word per TB rows, half the blocks past the last row and FP64 comparisons made the

@@ -879,7 +879,7 @@ struct astg_handle {
     // ---- several right-hand sides of one matrix (astg_solve_batch).  The matrix, its MIC(0) factor
     // and the level schedule are computed once and shared; each lane owns the PCG's vectors and
     // scalars and a stream and runs the launches astg_solve runs, so every solution is the one
-    // astg_solve returns, bit for bit.  A solve keeps one 16-CTA cluster busy in its
+    // astg_solve returns, bit for bit.  A solve keeps one cluster of at most 16 CTAs busy in its
     // preconditioner, so lanes on other SMs use the GPU that a single solve leaves idle; lanes are
     // driven by one host thread each.
     struct Lane {
@@ -955,13 +955,11 @@ struct astg_handle {
         ck(cudaMemcpyAsync(J.col, col, sizeof(int) * nnz, cudaMemcpyHostToDevice, st), "upload");
         ck(cudaMemcpyAsync(J.val, val, sizeof(double) * nnz, cudaMemcpyHostToDevice, st), "upload");
         select_preconditioner(J, n);
-        // more right-hand sides than such solves fit side by side: the form that shares SMs, if it does
-        if (J.pcAsync) {
-            const bool fp32 = precision == ASTG_MIXED && J.pcActive32;
-            const int alone = precond_concurrency(J, fp32);
-            if (nrhs > alone) select_preconditioner(J, n, true);
-            if (nrhs > alone && precond_concurrency(J, fp32) <= alone) select_preconditioner(J, n);
-        }
+        // more right-hand sides than such solves fit side by side: the form that shares SMs (20 right-hand
+        // sides, ms: 42 k rows 34 -> 28; from 100 k rows on, where a solve fills its SMs' shared memory
+        // and the L2, it is the slower one: 315 k rows FP64 230 -> 347)
+        if (J.pcAsync && n <= 100000 && nrhs > precond_concurrency(J, precision == ASTG_MIXED && J.pcActive32))
+            select_preconditioner(J, n, true);
         launch_external_system(d, J, n, st);
         checkStatus();
         bool mixed = precision == ASTG_MIXED && J.pcActive32;

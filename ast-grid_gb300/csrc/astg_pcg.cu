@@ -1553,6 +1553,9 @@ k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const in
                     }
                 }
                 const T y = acc * row.invd;
+                // spare lanes repeat a row, and z is the right-hand side of the backward sweep: every
+                // lane has read before any writes, also in an item without entries to wait for
+                __syncwarp();
                 K::st(own + (row.f & 0xffffffu) * (uint32_t)sizeof(T), y);
                 z[row.j] = y;
             }

@@ -57,3 +57,22 @@ def assert_same(name, ref, got, rel=0.0):
     else:
         r = max_rel(ref, got)
         assert r <= rel, f"{name}: max relative difference {r:.3e} > {rel:.1e}"
+
+
+def csr(n, pairs, diag):
+    """Symmetric CSR (rowptr, col, val) with -1 at `pairs` of rows and the row's count of them plus
+    `diag` (a number or one per row) on the diagonal."""
+    pairs = np.asarray(pairs, dtype=np.int64).reshape(-1, 2)
+    k = np.arange(n)
+    i, j = np.concatenate([pairs[:, 0], pairs[:, 1], k]), np.concatenate([pairs[:, 1], pairs[:, 0], k])
+    v = np.concatenate([-np.ones(2 * len(pairs)), np.bincount(pairs.ravel(), minlength=n) + diag])
+    o = np.lexsort((j, i))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(i, minlength=n))])
+    return rp.astype(np.int32), j[o].astype(np.int32), v[o]
+
+
+def residual(rp, col, val, x, b):
+    """The largest |b - A x|."""
+    r = np.array(b)
+    np.subtract.at(r, np.repeat(np.arange(len(b)), np.diff(rp)), val * x[col])
+    return np.abs(r).max()

@@ -2205,6 +2205,7 @@ __global__ void __cluster_dims__(SPMV_CTAS, 1, 1) __launch_bounds__(SPMV_THREADS
         double acc = 0.0;
         for (int k = 0; k < RED_PER_LANE && i + RED_LANES * k < n; ++k) acc = mac_add<FUSED>(acc, (double)ss[lane + 32 * k], (double)ys[lane + 32 * k]);
         *cg::this_cluster().map_shared_rank(sh + 32 * rank + lane, 0) = acc;
+        __syncwarp();  // the lanes' rows end at different k: together again for the aligned barrier
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     if (rank != 0) return;

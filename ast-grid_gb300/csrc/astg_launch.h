@@ -129,21 +129,21 @@ struct Proj {
     int pcWarps;     // warps per CTA
     int pcBlock;     // rows per ownership block
     int pcChunk;     // shared-memory slots per CTA (without the one that holds 0)
-    int itemCap;     // items, and quads after the first, that the arrays hold per sweep
+    int quadCap;     // quads after the first that the arrays hold per sweep
     int* itemTotal;  // device: items, forward and backward quads after the first
     int* ownCnt;     // pcCluster * (rows + 1): rows per segment
     int* ownPtr;     // first row of each segment in perm
     int* ownFill;
     int* itemPtr;    // first item of each segment
     int* permD[2];   // rows of each segment by descending entry count
-    int2* itemRange[2];  // first row in permD, rows
-    int* itXq[2];    // first quad after the first, per item
-    int4* itRow[2];  // row records, 32 per item (FP64)
+    int4* itDesc[2]; // rows (items at most): first position in permD, rows, first quad after the first,
+                     // quads | (entries of the first quad - 1) << 4 | any entry in another CTA << 7
+    int4* itRow[2];  // row records by position in permD (FP64)
     int4* itRow32[2];
-    int4* itCol[2];  // first quads, 32 per item
+    int4* itCol[2];  // first quads by position in permD
     double* itVal[2];
     float* itVal32[2];
-    int4* itXcol[2];  // quads after the first
+    int4* itXcol[2];  // quads after the first: per item, one per row for each
     double* itXval[2];
     float* itXval32[2];
     // mixed precision: FP32 copy of the matrix, FP32 inner vectors

@@ -1261,14 +1261,16 @@ __global__ void __launch_bounds__(256, 1) k_precond_dsmem(Proj P, double* z, int
 // returns a quiet NaN), and a single aligned store makes the value visible, so no separate flag is
 // needed.
 //
-// The rows of one CTA and level are sorted by their entry count and cut into items of 32 rows, one
-// per lane; item k of a CTA's walk belongs to its warp k mod W.  An item's records are stored for
-// the warp that reads them: one 16-byte row record per lane, then its entries four at a time (a
-// quad: four packed columns, four factor values), right-aligned, so that a row shorter than the
-// item's longest starts with entries of value 0 that read a slot holding 0 (fma(-0, 0, acc) = acc).
-// Every load is one coalesced 16-byte load per lane with no branch on the row's length, the next
-// item's records are fetched while this one waits, and the rows of an item are of one level, so
-// their lanes become ready together and the arithmetic runs once for the whole warp.
+// The rows of one CTA and level are sorted by their entry count and cut into items of up to 32 rows,
+// one per lane (spare lanes repeat the last); item k of a CTA's walk belongs to its warp k mod W.  An
+// item's records are stored for the warp that reads them: one 16-byte row record per row, then its
+// entries four at a time (a quad: four packed columns, four factor values), right-aligned, so that a
+// row shorter than the item's longest starts with entries of value 0 that read a slot holding 0
+// (fma(-0, 0, acc) = acc).  Records take space per row, none per spare lane: levels of a few rows
+// (chains, dense bands) need no more than wide ones.  Every load is one coalesced 16-byte load per
+// lane with no branch on the row's length, the next item's records (and the description of the one
+// after it) are fetched while this one waits, and the rows of an item are of one level, so their lanes
+// become ready together and the arithmetic runs once for the whole warp.
 //
 // Deadlock cannot occur: every warp walks its items in non-decreasing level order, rows read only
 // rows of strictly lower levels (forward) or higher levels (backward, walked in reverse), and all
@@ -1362,18 +1364,17 @@ __device__ __forceinline__ int4 ld_rec(const void* p) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
-// row record of an item's lane: pivot reciprocal, row, local slot | quads << 24 | (entries of the
-// first quad - 1) << 28 | any entry in another CTA << 31 (the last three are the item's)
+// row record: pivot reciprocal, row, local slot
 template <typename T> struct PcaRow;
 template <> struct alignas(16) PcaRow<double> {
     double invd;
     int j;
-    unsigned f;
+    int slot;
 };
 template <> struct alignas(16) PcaRow<float> {
     float invd;
     int j;
-    unsigned f;
+    int slot;
     int pad;
 };
 static_assert(sizeof(PcaRow<double>) == 16 && sizeof(PcaRow<float>) == 16, "row records are one 16-byte load");
@@ -1459,13 +1460,13 @@ __device__ __forceinline__ T pca_chain(T acc, int w, const PcaQuad<T>& q, const 
         if (w >= 4 - e) acc = sweep_update(true, acc, q.v[e], Pca<T>::val(s.z[e]));
     return acc;
 }
-// One sweep's items: row records and first quads at (item * 32 + lane), the quads after the first at
-// ((xq[item] + q - 1) * 32 + lane)
+// One sweep's items (Proj::itDesc): row records and first quads at the item's first position + lane, the
+// quads after the first at its first quad + (q - 1) * rows + lane
 template <typename T> struct PcaDir {
+    const int4* desc;
     const PcaRow<T>* row;
     const int4* col;
     const T* val;
-    const int* xq;
     const int4* xcol;
     const T* xval;
 };
@@ -1503,30 +1504,35 @@ k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const in
         // forward: the residual; backward: the forward sweep's result, written by this CTA
         const T* rhs = dir == 0 ? r : z;
         if (wid < items) {
-            size_t at = (size_t)(first + wid) * 32 + lane;
+            const int last = first + items - 1;
+            int4 d = __ldg(S.desc + first + wid), dn = __ldg(S.desc + min(first + wid + W, last));
+            size_t at = (size_t)d.x + min(lane, d.y - 1);
             PcaRow<T> m = pca_row(S.row + at);
             PcaQuad<T> q;
             pca_fetch(q, S.col, S.val, at);
-            int xq = __ldg(S.xq + first + wid);
 #pragma unroll 1
             for (int k = wid; k < items; k += W) {
                 const PcaRow<T> row = m;
                 const PcaQuad<T> q1 = q;
-                const size_t x = (size_t)xq * 32 + lane;
-                const unsigned f = __shfl_sync(0xffffffffu, row.f, 0) >> 24;
-                const int nq = f & 15, w0 = ((f >> 4) & 3) + 1;
+                // the item's flags through a shuffle: the compiler then knows them uniform and the branches
+                // on them cost nothing (loaded by every lane: 33 -> 39 us at 6 k rows)
+                const int f = __shfl_sync(0xffffffffu, d.w, 0);
+                const int nq = f & 15, w0 = ((f >> 4) & 3) + 1, xs = d.y;
                 const bool remote = (f & 128) != 0;
+                const size_t x = (size_t)d.z + min(lane, d.y - 1);
                 PcaVals<T> s1, s2, s3;
+                d = dn;  // past the last item: that one again
+                int p = d.x + min(lane, d.y - 1), k2 = min(first + k + 2 * W, last);
+                asm volatile("" : "+r"(p), "+r"(k2));  // ready before the look: no wait for its loads
                 if (nq > 0) pca_look(q1, s1, own, winA, remote);
                 asm volatile("" ::: "memory");  // the fetches below stay behind the use of q1
                 T acc = rhs[row.j];
-                const int kn = k + W < items ? k + W : k;  // the last item fetches itself again
-                at = (size_t)(first + kn) * 32 + lane;
+                at = (size_t)p;
                 m = pca_row(S.row + at);
-                xq = __ldg(S.xq + first + kn);
+                dn = __ldg(S.desc + k2);
                 PcaQuad<T> q2, q3;
                 if (nq > 1) pca_fetch(q2, S.xcol, S.xval, x);
-                if (nq > 2) pca_fetch(q3, S.xcol, S.xval, x + 32);
+                if (nq > 2) pca_fetch(q3, S.xcol, S.xval, x + xs);
                 pca_fetch(q, S.col, S.val, at);
                 if (nq > 0) {
                     pca_wait(s1, status);
@@ -1544,7 +1550,7 @@ k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const in
                         for (int e = 0; e < 4; ++e) acc = sweep_update(UNFUSED, acc, q3.v[e], K::val(s3.z[e]));
 #pragma unroll 1
                         for (int u = 2; u < nq - 1; ++u) {  // rows of more than 12 entries
-                            pca_fetch(q2, S.xcol, S.xval, x + 32 * (size_t)u);
+                            pca_fetch(q2, S.xcol, S.xval, x + (size_t)xs * u);
                             pca_look(q2, s2, own, winA, remote);
                             pca_wait(s2, status);
 #pragma unroll
@@ -1556,7 +1562,7 @@ k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const in
                 // spare lanes repeat a row, and z is the right-hand side of the backward sweep: every
                 // lane has read before any writes, also in an item without entries to wait for
                 __syncwarp();
-                K::st(own + (row.f & 0xffffffu) * (uint32_t)sizeof(T), y);
+                K::st(own + (uint32_t)row.slot * (uint32_t)sizeof(T), y);
                 z[row.j] = y;
             }
         }
@@ -1632,7 +1638,7 @@ static cudaError_t launch_precond_async(const Dev& d, const Proj& P, const PcaDa
 static PcaData<double> pca_data64(const Proj& P) {
     PcaData<double> D{};
     for (int k = 0; k < 2; ++k)
-        D.d[k] = PcaDir<double>{(const PcaRow<double>*)P.itRow[k], P.itCol[k], P.itVal[k], P.itXq[k], P.itXcol[k], P.itXval[k]};
+        D.d[k] = PcaDir<double>{P.itDesc[k], (const PcaRow<double>*)P.itRow[k], P.itCol[k], P.itVal[k], P.itXcol[k], P.itXval[k]};
     D.itemPtr = P.itemPtr;
     D.nLevels = P.nLevels;
     D.chunk = P.pcChunk;
@@ -1819,7 +1825,6 @@ __global__ void k_seg_sort(Proj P, int dir) {
     __shared__ int bins[8][ROW_W];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nl = *P.nLevels;
     const long long keys = (long long)P.pcCS * nl;
-    if (P.itemTotal[0] > P.itemCap) return;
     for (long long k = (long long)blockIdx.x * 8 + w; k < keys; k += (long long)gridDim.x * 8) {
         const int p0 = P.ownPtr[k], m = P.ownPtr[k + 1] - p0;
         if (m == 0) continue;
@@ -1846,72 +1851,65 @@ __global__ void k_seg_sort(Proj P, int dir) {
         const int n = (m + 31) >> 5;
         const int cta = (int)(k / nl);
         const int id0 = dir == 0 ? P.itemPtr[k] : P.itemPtr[(long long)cta * nl] + P.itemPtr[(long long)(cta + 1) * nl] - P.itemPtr[k] - n;
-        for (int u = lane; u < n; u += 32) P.itemRange[dir][id0 + u] = make_int2(p0 + 32 * u, min(32, m - 32 * u));
+        for (int u = lane; u < n; u += 32) P.itDesc[dir][id0 + u] = make_int4(p0 + 32 * u, min(32, m - 32 * u), 0, 0);
         __syncwarp();
     }
 }
-// one warp per item: the records of its 32 lanes (lanes past its last row repeat that row)
+// one warp per item: the records of its rows
 __global__ void k_item_fill(Proj P, int dir) {
-    const int item = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    const int total = P.itemTotal[0];
-    if (total > P.itemCap || item >= total) return;
-    const int2 rg = P.itemRange[dir][item];
-    const int i = P.permD[dir][rg.x + min(lane, rg.y - 1)];
-    const int dg = P.diagPos[i];
-    const int q0 = dir == 0 ? P.rowPtr[i] : dg + 1, q1 = dir == 0 ? dg : P.rowPtr[i + 1];
-    const int cnt = q1 - q0;
-    const int longest = __reduce_max_sync(0xffffffffu, cnt);
-    const int nq = (longest + 3) >> 2, w0 = nq ? longest - 4 * (nq - 1) : 1;
-    int x = 0;
-    if (nq > 1) {
-        if (lane == 0) x = atomicAdd(P.itemTotal + 1 + dir, nq - 1);
-        x = __shfl_sync(0xffffffffu, x, 0);
-        if (x + nq - 1 > P.itemCap) return;  // the host reads the totals and takes another form
-    }
-    if (lane == 0) P.itXq[dir][item] = x;
-    const int self = own_of(P, i);
-    bool remote = false;
-    for (int u = 0; u < max(nq, 1); ++u) {
-        int c[4];
-        double v[4];
-        for (int e = 0; e < 4; ++e) {
-            const int q = q0 + 4 * u + e - (4 * nq - cnt);  // right-aligned
-            c[e] = P.pcChunk;
-            v[e] = 0;
-            if (u < nq && q >= q0 && q < q1) {
-                const int k = P.col[q], o = own_of(P, k);
-                c[e] = slot_of(P, k);
-                if (o != self) {
-                    c[e] |= (o << 24) | (int)0x80000000u;
-                    remote = true;
-                }
-                v[e] = dir == 0 ? P.Lv[P.tpos[q]] : P.Lv[q];
-            }
+    const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * blockDim.x) >> 5, total = P.itemTotal[0];
+    for (int item = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < total; item += warps) {
+        int4 d = P.itDesc[dir][item];
+        const size_t first = (size_t)d.x + min(lane, d.y - 1);
+        const int i = P.permD[dir][first];
+        const int dg = P.diagPos[i];
+        const int q0 = dir == 0 ? P.rowPtr[i] : dg + 1, q1 = dir == 0 ? dg : P.rowPtr[i + 1];
+        const int cnt = q1 - q0;
+        const int longest = __reduce_max_sync(0xffffffffu, cnt);
+        const int nq = (longest + 3) >> 2, w0 = nq ? longest - 4 * (nq - 1) : 1;
+        if (nq > 1) {
+            if (lane == 0) d.z = atomicAdd(P.itemTotal + 1 + dir, (nq - 1) * d.y);
+            d.z = __shfl_sync(0xffffffffu, d.z, 0);
+            if (d.z + (nq - 1) * d.y > P.quadCap) continue;  // the host reads the totals
         }
-        const size_t at = (size_t)(u == 0 ? item : x + u - 1) * 32 + lane;
-        (u == 0 ? P.itCol : P.itXcol)[dir][at] = make_int4(c[0], c[1], c[2], c[3]);
-        double2* dv = reinterpret_cast<double2*>((u == 0 ? P.itVal : P.itXval)[dir] + 4 * at);
-        dv[0] = make_double2(v[0], v[1]);
-        dv[1] = make_double2(v[2], v[3]);
-        // the factor is computed in FP64 and rounded once
-        *reinterpret_cast<float4*>((u == 0 ? P.itVal32 : P.itXval32)[dir] + 4 * at) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+        const int self = own_of(P, i);
+        bool remote = false;
+        for (int u = 0; u < max(nq, 1); ++u) {
+            int c[4];
+            double v[4];
+            for (int e = 0; e < 4; ++e) {
+                const int q = q0 + 4 * u + e - (4 * nq - cnt);  // right-aligned
+                c[e] = P.pcChunk;
+                v[e] = 0;
+                if (u < nq && q >= q0 && q < q1) {
+                    const int k = P.col[q], o = own_of(P, k);
+                    c[e] = slot_of(P, k);
+                    if (o != self) {
+                        c[e] |= (o << 24) | (int)0x80000000u;
+                        remote = true;
+                    }
+                    v[e] = dir == 0 ? P.Lv[P.tpos[q]] : P.Lv[q];
+                }
+            }
+            if (lane >= d.y) continue;
+            const size_t at = u == 0 ? first : (size_t)d.z + (size_t)(u - 1) * d.y + lane;
+            (u == 0 ? P.itCol : P.itXcol)[dir][at] = make_int4(c[0], c[1], c[2], c[3]);
+            double2* dv = reinterpret_cast<double2*>((u == 0 ? P.itVal : P.itXval)[dir] + 4 * at);
+            dv[0] = make_double2(v[0], v[1]);
+            dv[1] = make_double2(v[2], v[3]);
+            // the factor is computed in FP64 and rounded once
+            *reinterpret_cast<float4*>((u == 0 ? P.itVal32 : P.itXval32)[dir] + 4 * at) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+        }
+        d.w = nq | ((w0 - 1) << 4) | (__any_sync(0xffffffffu, remote) ? 128 : 0);
+        if (lane == 0) P.itDesc[dir][item] = d;
+        if (lane < d.y) {
+            ((PcaRow<double>*)P.itRow[dir])[first] = PcaRow<double>{P.invdiag[i], i, slot_of(P, i)};
+            ((PcaRow<float>*)P.itRow32[dir])[first] = PcaRow<float>{(float)P.invdiag[i], i, slot_of(P, i), 0};
+        }
     }
-    const unsigned f = (unsigned)slot_of(P, i) | ((unsigned)(nq | ((w0 - 1) << 4) | (__any_sync(0xffffffffu, remote) ? 128 : 0)) << 24);
-    const size_t at = (size_t)item * 32 + lane;
-    PcaRow<double> r;
-    r.invd = P.invdiag[i];
-    r.j = i;
-    r.f = f;
-    ((PcaRow<double>*)P.itRow[dir])[at] = r;
-    PcaRow<float> r32;
-    r32.invd = (float)P.invdiag[i];
-    r32.j = i;
-    r32.f = f;
-    r32.pad = 0;
-    ((PcaRow<float>*)P.itRow32[dir])[at] = r32;
 }
-// false when the items do not fit their arrays (a matrix of very many, very narrow levels): the
-// caller takes another form of the sweeps
+// false when the quads after the first do not fit their arrays (rows far longer than others of their
+// item): the caller takes another form of the sweeps
 static bool launch_item_schedule(Proj& P, cudaStream_t st) {
     const int maxRows = P.rows;
     cudaMemsetAsync(P.nLevels, 0, sizeof(int), st);
@@ -1922,12 +1920,12 @@ static bool launch_item_schedule(Proj& P, cudaStream_t st) {
     ASTG_LAUNCH(k_seg_scatter<<<nblk(maxRows), TB, 0, st>>>(P));
     for (int dir = 0; dir < 2; ++dir) {
         ASTG_LAUNCH(k_seg_sort<<<512, TB, 0, st>>>(P, dir));
-        ASTG_LAUNCH(k_item_fill<<<nblk((long long)P.itemCap * 32), TB, 0, st>>>(P, dir));
+        ASTG_LAUNCH(k_item_fill<<<std::min(nblk(32LL * maxRows), 152 * 8), TB, 0, st>>>(P, dir));
     }
     int total[3] = {0, 0, 0};
     cudaMemcpyAsync(total, P.itemTotal, sizeof total, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
-    return total[0] <= P.itemCap && total[1] <= P.itemCap && total[2] <= P.itemCap;
+    return total[1] <= P.quadCap && total[2] <= P.quadCap;
 }
 
 void launch_level_schedule(const Dev& d, Proj& P, bool owner, cudaStream_t st) {
@@ -2870,7 +2868,7 @@ __global__ void k_mixed_finish(Proj P, double res, double tolAbs, double res0, i
 static PcaData<float> pca_data32(const Proj& P) {
     PcaData<float> D{};
     for (int k = 0; k < 2; ++k)
-        D.d[k] = PcaDir<float>{(const PcaRow<float>*)P.itRow32[k], P.itCol[k], P.itVal32[k], P.itXq[k], P.itXcol[k], P.itXval32[k]};
+        D.d[k] = PcaDir<float>{P.itDesc[k], (const PcaRow<float>*)P.itRow32[k], P.itCol[k], P.itVal32[k], P.itXcol[k], P.itXval32[k]};
     D.itemPtr = P.itemPtr;
     D.nLevels = P.nLevels;
     D.chunk = P.pcChunk;
@@ -3037,22 +3035,20 @@ void proj_alloc(Proj& J, long long rows, int device, cudaStream_t st, std::vecto
     J.pcSmem = 0;
     J.bsum = A.get<int>((rows * ROW_W + 1 + 1023) / 1024 + 1);
     if (J.pcCluster && J.pcAsync) {
-        // items: 32 rows each where levels are wide, at least one per level and CTA; a sixteenth of the
-        // rows is twice what the octree systems take (all of them on small handles)
-        J.itemCap = (int)std::max(std::min(rows, 32768LL), rows / 16);
-        const long long L = 32LL * J.itemCap;
+        // the quads after the first share the memory of the level-order entries (a solve uses one of the
+        // two): four a row, and with the n * 31 / 2 entries that a sweep can have rows need no more
+        J.quadCap = (int)(rows * (ROW_W / 8));
         for (int k = 0; k < 2; ++k) {
             J.permD[k] = A.get<int>(rows);
-            J.itemRange[k] = A.get<int2>(J.itemCap);
-            J.itXq[k] = A.get<int>(J.itemCap);
-            J.itRow[k] = A.get<int4>(L);
-            J.itRow32[k] = A.get<int4>(L);
-            J.itCol[k] = A.get<int4>(L);
-            J.itXcol[k] = A.get<int4>(L);
-            J.itVal[k] = A.get<double>(4 * L);
-            J.itXval[k] = A.get<double>(4 * L);
-            J.itVal32[k] = A.get<float>(4 * L);
-            J.itXval32[k] = A.get<float>(4 * L);
+            J.itDesc[k] = A.get<int4>(rows);
+            J.itRow[k] = A.get<int4>(rows);
+            J.itRow32[k] = A.get<int4>(rows);
+            J.itCol[k] = A.get<int4>(rows);
+            J.itVal[k] = A.get<double>(4 * rows);
+            J.itVal32[k] = A.get<float>(4 * rows);
+            J.itXcol[k] = (int4*)(k ? J.bcol : J.fcol);
+            J.itXval[k] = k ? J.bval : J.fval;
+            J.itXval32[k] = A.get<float>(4LL * J.quadCap);
         }
         J.itemTotal = A.get<int>(3);
         J.ownCnt = A.get<int>((rows + 1) * J.pcCluster);

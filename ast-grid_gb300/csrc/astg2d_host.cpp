@@ -190,7 +190,6 @@ struct astg2_handle {
         } else {
             bool owner = mixed || (J.pcActive && J.pcAsync);
             if (J.clusterSize > 0 || J.pcActive || mixed) launch_level_schedule(d, J, owner, st);
-            mixed = mixed && J.pcActive32;
         }
         if (mixed) launch_pcg_mixed(d, J, tol, maxIter, 8, st, &prof);
         else launch_pcg_fp64(d, J, tol, maxIter, epoch, 8, st, &prof);

@@ -497,11 +497,10 @@ struct astg_handle {
     // factorises the system held in the projection workspace and runs the PCG (mixed precision
     // when asked for and the FP32 preconditioner fits, else FP64); J.x holds the result
     void solveCurrent(double tol, int maxIter, int precision) {
-        bool mixed = precision == ASTG_MIXED && J.pcActive32;
+        const bool mixed = precision == ASTG_MIXED && J.pcActive32;
         launch_factor(d, J, P.omega, P.min_diag, epoch, st, &prof);
         bool owner = mixed || (J.pcActive && J.pcAsync);
         if (J.clusterSize > 0 || J.pcActive || mixed) launch_level_schedule(d, J, owner, st);
-        mixed = mixed && J.pcActive32;
         ck(cudaEventRecord(evA, st), "event");
         lastOuter = 0;
         if (mixed) lastOuter = launch_pcg_mixed(d, J, tol, maxIter, 8, st, &prof);
@@ -962,11 +961,10 @@ struct astg_handle {
             select_preconditioner(J, n, true);
         launch_external_system(d, J, n, st);
         checkStatus();
-        bool mixed = precision == ASTG_MIXED && J.pcActive32;
+        const bool mixed = precision == ASTG_MIXED && J.pcActive32;
         launch_factor(d, J, P.omega, P.min_diag, epoch, st, nullptr);
         const bool owner = mixed || (J.pcActive && J.pcAsync);
         if (J.clusterSize > 0 || J.pcActive || mixed) launch_level_schedule(d, J, owner, st);
-        mixed = mixed && J.pcActive32;
         ck(cudaStreamSynchronize(st), "factor");
         checkStatus();
         // lanes only with the barrier-free preconditioner: the other forms hand rows out from one

@@ -130,6 +130,8 @@ struct Proj {
     int pcBlock;     // rows per ownership block
     int pcChunk;     // shared-memory slots per CTA (without the one that holds 0)
     int quadCap;     // quads after the first that the arrays hold per sweep
+    int quadsGrown;  // 1: the arrays of those quads are their own (grow_quads)
+    std::vector<void*>* owned;  // host: the handle's device allocations
     int* itemTotal;  // device: items, forward and backward quads after the first
     int* ownCnt;     // pcCluster * (rows + 1): rows per segment
     int* ownPtr;     // first row of each segment in perm
@@ -266,8 +268,7 @@ void launch_velocity_ghost(const Dev& d, const Fields& F, const uint8_t* lastWri
 void launch_dof_numbering(const Dev& d, const uint8_t* open, Proj& P, cudaStream_t st);
 void launch_assemble(const Dev& d, const Fields& F, const uint8_t* open, Proj& P, const int* hoPtr, const int* hoIdx,
                      double dt, cudaStream_t st);
-// owner: the items of the barrier-free preconditioner, else the level order (also when the items do
-// not fit: P.pcActive and P.pcActive32 are then cleared)
+// owner: the items of the barrier-free preconditioner, else the level order
 void launch_level_schedule(const Dev& d, Proj& P, bool owner, cudaStream_t st);
 void launch_external_system(const Dev& d, Proj& P, int rows, cudaStream_t st);
 // padded rows (rowCnt, padCol, padVal, bRaw over maxRows rows, *nDof set) -> CSR with b = bRaw *

@@ -1908,9 +1908,56 @@ __global__ void k_item_fill(Proj P, int dir) {
         }
     }
 }
-// false when the quads after the first do not fit their arrays (rows far longer than others of their
-// item): the caller takes another form of the sweeps
-static bool launch_item_schedule(Proj& P, cudaStream_t st) {
+namespace {
+struct ProjArena {
+    cudaStream_t st;
+    std::vector<void*>& allocs;
+    void ck(cudaError_t e, const char* what) {
+        if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
+    }
+    template <class T>
+    T* get(long long n) {
+        void* p = nullptr;
+        size_t bytes = (size_t)std::max<long long>(n, 1) * sizeof(T);
+        ck(cudaMalloc(&p, bytes), "cudaMalloc");
+        allocs.push_back(p);
+        ck(cudaMemsetAsync(p, 0, bytes, st), "cudaMemset");
+        return (T*)p;
+    }
+    void release(void* p) {  // nothing on the device uses it any more
+        allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
+        cudaFree(p);
+    }
+};
+}  // namespace
+
+// Room for `need` quads after the first and a quarter more; a row has eight quads at most.  Matrices
+// whose items mix rows of very different lengths take this, once; the others fit what a handle has.
+static void grow_quads(Proj& P, int need, cudaStream_t st) {
+    ProjArena A{st, *P.owned};
+    const long long cap = std::min((long long)P.rowsCap * (ROW_W / 4 - 1), need + need / 4LL);
+    int4* xcol[2];
+    double* xval[2];
+    float* xval32[2];
+    for (int k = 0; k < 2; ++k) {
+        xcol[k] = A.get<int4>(cap);
+        xval[k] = A.get<double>(4 * cap);
+        xval32[k] = A.get<float>(4 * cap);
+    }
+    for (int k = 0; k < 2; ++k) {
+        A.release(P.itXval32[k]);
+        if (P.quadsGrown) {
+            A.release(P.itXcol[k]);
+            A.release(P.itXval[k]);
+        }
+        P.itXcol[k] = xcol[k];
+        P.itXval[k] = xval[k];
+        P.itXval32[k] = xval32[k];
+    }
+    P.quadsGrown = 1;
+    P.quadCap = (int)cap;
+}
+static void launch_item_schedule(Proj& P, cudaStream_t st) {
     const int maxRows = P.rows;
     cudaMemsetAsync(P.nLevels, 0, sizeof(int), st);
     ASTG_LAUNCH(k_seg_levels<<<std::min(nblk(maxRows), 512), TB, 0, st>>>(P));
@@ -1918,22 +1965,23 @@ static bool launch_item_schedule(Proj& P, cudaStream_t st) {
     ASTG_LAUNCH(k_seg_hist<<<nblk(maxRows), TB, 0, st>>>(P));
     ASTG_LAUNCH(k_seg_scan<<<1, 1024, 0, st>>>(P));
     ASTG_LAUNCH(k_seg_scatter<<<nblk(maxRows), TB, 0, st>>>(P));
-    for (int dir = 0; dir < 2; ++dir) {
-        ASTG_LAUNCH(k_seg_sort<<<512, TB, 0, st>>>(P, dir));
-        ASTG_LAUNCH(k_item_fill<<<std::min(nblk(32LL * maxRows), 152 * 8), TB, 0, st>>>(P, dir));
+    for (int dir = 0; dir < 2; ++dir) ASTG_LAUNCH(k_seg_sort<<<512, TB, 0, st>>>(P, dir));
+    for (;;) {
+        for (int dir = 0; dir < 2; ++dir) ASTG_LAUNCH(k_item_fill<<<std::min(nblk(32LL * maxRows), 152 * 8), TB, 0, st>>>(P, dir));
+        int total[3] = {0, 0, 0};
+        cudaMemcpyAsync(total, P.itemTotal, sizeof total, cudaMemcpyDeviceToHost, st);
+        cudaStreamSynchronize(st);
+        const int need = std::max(total[1], total[2]);
+        if (need <= P.quadCap) return;
+        grow_quads(P, need, st);
+        cudaMemsetAsync(P.itemTotal + 1, 0, 2 * sizeof(int), st);
     }
-    int total[3] = {0, 0, 0};
-    cudaMemcpyAsync(total, P.itemTotal, sizeof total, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    return total[1] <= P.quadCap && total[2] <= P.quadCap;
 }
 
 void launch_level_schedule(const Dev& d, Proj& P, bool owner, cudaStream_t st) {
     if (owner) {
-        if (launch_item_schedule(P, st)) return;
-        P.pcActive = 0;  // the level-synchronous sweeps, in level order
-        P.pcActive32 = 0;
-        if (P.clusterSize <= 0) return;
+        launch_item_schedule(P, st);
+        return;
     }
     const int maxRows = P.rows;
     ASTG_LAUNCH(k_level_reset<<<nblk(maxRows + 1), TB, 0, st>>>(P, maxRows));
@@ -2962,29 +3010,11 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
     return outer;
 }
 // ------------------------------------------------------------------ workspace
-namespace {
-struct ProjArena {
-    cudaStream_t st;
-    std::vector<void*>& allocs;
-    void ck(cudaError_t e, const char* what) {
-        if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
-    }
-    template <class T>
-    T* get(long long n) {
-        void* p = nullptr;
-        size_t bytes = (size_t)std::max<long long>(n, 1) * sizeof(T);
-        ck(cudaMalloc(&p, bytes), "cudaMalloc");
-        allocs.push_back(p);
-        ck(cudaMemsetAsync(p, 0, bytes, st), "cudaMemset");
-        return (T*)p;
-    }
-};
-}  // namespace
-
 void proj_alloc(Proj& J, long long rows, int device, cudaStream_t st, std::vector<void*>& allocs) {
     if (rows <= 0 || rows * ROW_W >= (1LL << 31)) throw std::runtime_error("projection too large for 32-bit matrix indices");
     ProjArena A{st, allocs};
     J.rowsCap = (int)rows;
+    J.owned = &allocs;
     J.n0 = A.get<int>(1);
     J.nDof = A.get<int>(1);
     J.nnz = A.get<int>(4);  // nnz, then scan totals of the level schedule
@@ -3036,7 +3066,8 @@ void proj_alloc(Proj& J, long long rows, int device, cudaStream_t st, std::vecto
     J.bsum = A.get<int>((rows * ROW_W + 1 + 1023) / 1024 + 1);
     if (J.pcCluster && J.pcAsync) {
         // the quads after the first share the memory of the level-order entries (a solve uses one of the
-        // two): four a row, and with the n * 31 / 2 entries that a sweep can have rows need no more
+        // two): four a row, more than the 31 / 2 entries a row that a sweep can have on average fill; an
+        // item whose rows differ much in length takes more (grow_quads)
         J.quadCap = (int)(rows * (ROW_W / 8));
         for (int k = 0; k < 2; ++k) {
             J.permD[k] = A.get<int>(rows);

@@ -56,3 +56,46 @@ def test_a_chain_keeps_the_precision_asked_for(n):
     assert sm.converged == 1 and sm.outer > 0 and residual(rp, col, val, xm, b) <= 1e-6 * np.abs(b).max() * (1 + 1e-6)
     s.close()
     o.close()
+
+
+def ladder(levels, width=32, reach=31):
+    """Levels of `width` rows: rows 1.. each on its namesake of the level before, row 0 on `reach` of
+    them.  Every item of 32 rows (forward) then holds one row of 31 entries and 31 of one."""
+    at = np.arange(1, levels)[:, None] * width
+    k = np.arange(1, width)[None, :]
+    same = np.stack([(at - width + k).ravel(), (at + k).ravel()], 1)
+    far = np.stack([(at - width + k[:, :reach]).ravel(), np.broadcast_to(at, (levels - 1, reach)).ravel()], 1)
+    return np.unique(np.concatenate([same, far]), axis=0)
+
+
+@pytest.mark.parametrize("share", [0.1, 0.5, 0.95])
+def test_items_of_rows_of_very_different_lengths(share):
+    """Seven quads after the first for each row of the forward sweep, where a handle starts with room for
+    four per row of its capacity: the largest share takes more (and the next solve finds it)."""
+    import ast_solver
+    from oracle.oracle import Oracle
+
+    s, o = ast_solver.OctreeSmoke3(16, 2), Oracle(8, 2, reduce_mode=1)
+    capacity = 2 * int(s.get("level_sizes")[:, 0].sum()) + len(s.get("half_tilts"))
+    levels = int(share * capacity) // 32
+    n = 32 * levels
+    rp, col, val = csr(n, ladder(levels), 0.05)
+    assert np.diff(rp).max() == 32
+    b = np.random.default_rng(n).standard_normal(n)
+    xo, ito = o.solve(rp, col, val, b)
+    for _ in range(2):
+        xm, sm = s.solve(rp, col, val, b, precision="mixed")
+        assert sm.converged == 1 and sm.outer > 0
+        assert residual(rp, col, val, xm, b) <= 1e-6 * np.abs(b).max() * (1 + 1e-6)
+        x, st = s.solve(rp, col, val, b)
+        assert st.converged == 1 and st.iterations == ito
+        np.testing.assert_array_equal(x, xo)
+    X = s.solve_batch(rp, col, val, np.stack([b, 2 * b, b]))[0]
+    np.testing.assert_array_equal(X[0], xo)
+    np.testing.assert_array_equal(X[2], xo)
+    s.update(0.01)  # the handle's own systems after the caller's
+    p = ast_solver.OctreeSmoke3(16, 2)
+    p.update(0.01)
+    np.testing.assert_array_equal(s.get("p"), p.get("p"))
+    for h in (s, p, o):
+        h.close()

@@ -851,8 +851,7 @@ void launch_precond_wave(const Proj& P, const double* r, double* z, cudaStream_t
     cudaLaunchAttribute at[1];
     wave_config(P.wnx, P.wny, st, cfg, at);
     count_launch();
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k2_precond_wave, P, r, z);
-    if (e != cudaSuccess) g_cluster_error = e;
+    note_launch(cudaLaunchKernelEx(&cfg, k2_precond_wave, P, r, z));
 }
 // The wavefront kernel takes up to WAVE_MAX_NX columns (16 CTAs of 32) and as many rows as fit a
 // CTA's shared memory; its slots use 32-bit indices.  Wider and taller grids take the generic sweeps.  Call with the device current.

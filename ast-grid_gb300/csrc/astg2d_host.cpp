@@ -201,11 +201,7 @@ struct astg2_handle {
         ck2(cudaMemcpyAsync(sc, J.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "stats");
         ck2(cudaMemcpyAsync(&nnz, J.nnz, sizeof nnz, cudaMemcpyDeviceToHost, st), "stats");
         ck2(cudaStreamSynchronize(st), "project");
-        if (g_cluster_error != cudaSuccess) {
-            cudaError_t e = g_cluster_error;
-            g_cluster_error = cudaSuccess;
-            ck2(e, "cluster sweep launch");
-        }
+        ck2(take_launch_error(), "PCG kernel launch");
         lastN = n;
         lastNnz = nnz;
         last.unknowns = n;

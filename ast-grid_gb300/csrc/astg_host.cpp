@@ -828,11 +828,7 @@ struct astg_handle {
         ck(cudaMemcpyAsync(&n, J.nDof, sizeof n, cudaMemcpyDeviceToHost, st), "stats");
         ck(cudaMemcpyAsync(&nnz, J.nnz, sizeof nnz, cudaMemcpyDeviceToHost, st), "stats");
         ck(cudaStreamSynchronize(st), "project");
-        if (g_cluster_error != cudaSuccess) {
-            cudaError_t e = g_cluster_error;
-            g_cluster_error = cudaSuccess;
-            ck(e, "cluster sweep launch");
-        }
+        ck(take_launch_error(), "PCG kernel launch");
         float ms = 0;
         cudaEventElapsedTime(&ms, evA, evB);
         last.iterations = isc[ISC_ITERS];
@@ -998,6 +994,7 @@ struct astg_handle {
                 ck(cudaMemcpyAsync(isc, J.isc, sizeof isc, cudaMemcpyDeviceToHost, st), "stats");
                 ck(cudaMemcpyAsync(sc, J.sc, sizeof sc, cudaMemcpyDeviceToHost, st), "stats");
                 ck(cudaStreamSynchronize(st), "solve");
+                ck(take_launch_error(), "PCG kernel launch");
                 float ms = 0;
                 cudaEventElapsedTime(&ms, evA, evB);
                 record(i, outer, isc, sc, ms);
@@ -1027,6 +1024,7 @@ struct astg_handle {
                             ck(cudaMemcpyAsync(isc, Q.isc, sizeof isc, cudaMemcpyDeviceToHost, L.st), "stats");
                             ck(cudaMemcpyAsync(sc, Q.sc, sizeof sc, cudaMemcpyDeviceToHost, L.st), "stats");
                             ck(cudaStreamSynchronize(L.st), "solve");
+                            ck(take_launch_error(), "PCG kernel launch");
                             float ms = 0;
                             cudaEventElapsedTime(&ms, L.e0, L.e1);
                             out[w].push_back({i, {(double)isc[ISC_ITERS], (double)isc[ISC_CONVERGED], (double)outer,
@@ -1048,11 +1046,6 @@ struct astg_handle {
                     sc[SC_TOL] = v[4];
                     record(rec.first, (int)v[2], isc, sc, (float)v[5]);
                 }
-        }
-        if (g_cluster_error != cudaSuccess) {
-            cudaError_t e = g_cluster_error;
-            g_cluster_error = cudaSuccess;
-            ck(e, "cluster sweep launch");
         }
         checkStatus();
         lastLanes = std::max(k, 1);
@@ -1275,6 +1268,7 @@ struct astg_handle {
         int it[2] = {0, 0};
         ck(cudaMemcpyAsync(it, J.isc, sizeof it, cudaMemcpyDeviceToHost, st), "iters");
         ck(cudaStreamSynchronize(st), "sync");
+        ck(take_launch_error(), "PCG kernel launch");
         ++adjSolves;
         adjIters += it[ISC_ITERS];
         launch_adj_rhs(d, C, g, dOpen, J, dHoPtr, dHoIdx, J.x, P.rho / dt, st);

@@ -285,7 +285,10 @@ int choose_cluster_size(int device);
 int choose_dsmem_cluster(bool async, size_t* smemMax);
 // per solve: whether the fused preconditioner holds a vector of n rows (sets pcActive, pcSmem)
 void select_preconditioner(Proj& P, int n, bool batch = false);
-extern cudaError_t g_cluster_error;  // last failed cluster launch (cudaSuccess if none)
+// the first PCG launch of this thread's current solve that was refused (cudaSuccess if none); taking it
+// clears it
+void note_launch(cudaError_t e);
+cudaError_t take_launch_error();
 void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epoch, cudaStream_t st, KProf* prof);
 // the wavefront preconditioner z = (L L^T)^-1 r of a uniform 2-D system (Proj::wave), astg2d.cu
 void launch_precond_wave(const Proj& P, const double* r, double* z, cudaStream_t st);

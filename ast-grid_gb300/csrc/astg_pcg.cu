@@ -47,6 +47,20 @@ namespace astg {
 std::atomic<long long> g_launches{0};
 thread_local long long t_launches = 0;
 
+// A refused launch leaves its kernel's outputs as they were and the solve would go on with them; each
+// PCG launch notes its result here, and whoever started the solve asks.  Per thread: handles and lanes
+// are driven by threads of their own.
+static thread_local cudaError_t t_launch_error = cudaSuccess;
+void note_launch(cudaError_t e) {
+    if (e != cudaSuccess && t_launch_error == cudaSuccess) t_launch_error = e;
+}
+cudaError_t take_launch_error() {
+    const cudaError_t e = t_launch_error;
+    t_launch_error = cudaSuccess;
+    if (e != cudaSuccess) cudaGetLastError();  // reported by the caller
+    return e;
+}
+
 // event pairs around profiled launches; drained after each host synchronisation.  On a capturing
 // stream the records become event-record nodes of the graph (external records) in a separate set
 // of pairs, which every replay records again.
@@ -123,6 +137,7 @@ struct BatchGraph {
     template <typename Body>
     bool run(Body body, int nb, cudaStream_t st, KProf* prof) {
         if (failed) return false;
+        const cudaError_t before = t_launch_error;  // a capture that fails is launched directly instead
         const int k = (prof && prof->on && replays % KPROF_GRAPH_EVERY == 0) ? 1 : 0;
         if (!exec[k]) {
             if (k) prof->gused = 0;
@@ -142,6 +157,7 @@ struct BatchGraph {
             t_launches -= launches[k];
             if (e != cudaSuccess) {
                 cudaGetLastError();
+                t_launch_error = before;
                 exec[k] = nullptr;
                 failed = true;
                 return false;
@@ -199,7 +215,7 @@ static void launch_pdl(void (*k)(KArgs...), int grid, int block, cudaStream_t st
     cfg.attrs = at;
     cfg.numAttrs = 1;
     count_launch();
-    cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+    note_launch(cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...));
 }
 
 // ------------------------------------------------------------------ fixed-tree reduction
@@ -1090,7 +1106,6 @@ __global__ void k_level_reset(Proj P, int rows) {
 // ------------------------------------------------------------------ cluster sweeps
 constexpr int CLUSTER_THREADS = 512;
 constexpr int PC_THREADS = 256;
-cudaError_t g_cluster_error = cudaSuccess;
 // One thread-block cluster walks the levels; a hardware cluster barrier (release/acquire at
 // cluster scope) separates consecutive levels, so no row ever polls a flag.  Per row the
 // operations are the reference's, in the same order.
@@ -2552,7 +2567,7 @@ static void precond(const Dev& d, Proj& P, const double* r, double* z, int& epoc
         cudaError_t e = P.pcAsync ? launch_precond_async(d, P, pca_data64(P), r, z, P.pcSmem, st)
                                   : launch_precond_dsmem(P, r, z, st);
         prof_end(prof, st);
-        if (e != cudaSuccess) g_cluster_error = e;
+        note_launch(e);
         return;
     }
     if (P.clusterSize > 0) {
@@ -2562,8 +2577,8 @@ static void precond(const Dev& d, Proj& P, const double* r, double* z, int& epoc
         prof_begin(prof, 1, st);
         cudaError_t e2 = launch_cluster(k_sweep_bwd_cluster, P.clusterSize, st, P, nullptr, z);
         prof_end(prof, st);
-        if (e != cudaSuccess) g_cluster_error = e;
-        if (e2 != cudaSuccess) g_cluster_error = e2;
+        note_launch(e);
+        note_launch(e2);
         return;
     }
     int warps = P.sweepBlocks;
@@ -2762,6 +2777,7 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
     double* r = P.r;
     double* s = P.s;
     double* z = P.z;
+    t_launch_error = cudaSuccess;
     const int rowBlocks = update_blocks(maxRows);
     ASTG_LAUNCH(k_zero_vec<<<nblk(maxRows), TB, 0, st>>>(x, P.nDof));
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(P.b, r, P.nDof));
@@ -2825,7 +2841,7 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
         cudaStreamSynchronize(st);
         prof_drain(prof, replayed && graph.profiled);
         hostDone = *P.hostDone;
-        if (hostDone) break;
+        if (hostDone || t_launch_error != cudaSuccess) break;
     }
     return launched;
 }
@@ -2936,6 +2952,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
     int chunks = (maxRows + RED_CHUNK - 1) / RED_CHUNK;
     double* x = P.x;
     double* r = P.r;
+    t_launch_error = cudaSuccess;
     const int rowBlocks = update_blocks(maxRows);
     ASTG_LAUNCH(k_zero_vec<<<nblk(maxRows), TB, 0, st>>>(x, P.nDof));
     ASTG_LAUNCH(k_copy<<<nblk(maxRows), TB, 0, st>>>(P.b, r, P.nDof));
@@ -2964,7 +2981,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
         prof_begin(prof, 0, st);
         cudaError_t e = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
         prof_end(prof, st);
-        if (e != cudaSuccess) g_cluster_error = e;
+        note_launch(e);
         launch_pdl(k_dot_zr<float, false, false>, chunks, RED_LANES, st, P, P.z32, P.r32, P.part);
         ASTG_LAUNCH(k_inner_start<<<1, RED_LANES, 0, st>>>(P, P.part, innerTol));
         ASTG_LAUNCH(k_copy32<<<nblk(maxRows), TB, 0, st>>>(P.z32, P.s32, P.nDof));
@@ -2973,7 +2990,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
             for (int it = 0; it < nb; ++it) {
                 if (mid) {
                     cudaError_t pe = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
-                    if (pe != cudaSuccess) g_cluster_error = pe;
+                    note_launch(pe);
                     launch_pdl(k_mid<float, false>, MID_CTAS, MID_THREADS, st, P, P.e32, P.r32, P.s32, (const float*)P.z32, maxIter);
                     continue;
                 }
@@ -2984,7 +3001,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
                 prof_begin(pf, 0, st);
                 cudaError_t pe = launch_precond_async(d, P, D, (const float*)P.r32, P.z32, P.pcSmem32, st);
                 prof_end(pf, st);
-                if (pe != cudaSuccess) g_cluster_error = pe;
+                note_launch(pe);
                 launch_pdl(k_dot_zr<float, false, true>, chunks, RED_LANES, st, P, P.z32, P.r32, P.part);
                 launch_pdl(k_update_s32, nblk(maxRows), TB, st, P);
             }
@@ -2996,8 +3013,9 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
             cudaMemcpyAsync(P.hostDone, P.done, sizeof(int), cudaMemcpyDeviceToHost, st);
             cudaStreamSynchronize(st);
             prof_drain(prof, replayed && graph.profiled);
-            if (*P.hostDone) break;
+            if (*P.hostDone || t_launch_error != cudaSuccess) break;
         }
+        if (t_launch_error != cudaSuccess) break;
         ASTG_LAUNCH(k_add_correction<<<nblk(maxRows), TB, 0, st>>>(P, x));
         cudaMemsetAsync(P.amax, 0, sizeof(unsigned long long), st);
         prof_begin(prof, 2, st);

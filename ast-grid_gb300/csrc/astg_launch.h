@@ -122,6 +122,8 @@ struct Proj {
     double* fvalP;
     int* bcolP;
     double* bvalP;
+    int midRuns;     // the device runs k_mid's cluster
+    int spmvCluster; // the product over clusters, else one CTA per chunk (k_spmv_dot_block)
     int pcAsync;     // 1: barrier-free fused preconditioner, 0: one cluster barrier per level
     // barrier-free form (k_precond_async): rows dealt to pcCS CTAs in blocks of pcBlock, the rows of a
     // (CTA, level) segment cut into items of 32; [0] forward, [1] backward

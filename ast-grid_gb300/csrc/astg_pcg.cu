@@ -1659,7 +1659,6 @@ static PcaData<double> pca_data64(const Proj& P) {
     D.chunk = P.pcChunk;
     return D;
 }
-static void allow_mid_clusters();
 // Cluster size (16, else 8) at which the fused preconditioner (barrier-free form when async) can
 // run with the largest dynamic shared memory a CTA may have, or 0; *smemMax = that largest size.
 // Each solve then uses ceil(n / CS) doubles per CTA and falls back to the global-memory sweeps
@@ -1669,7 +1668,6 @@ int choose_dsmem_cluster(bool async, size_t* smemMax) {
     const int threads = async ? PCA_MAX_WARPS * 32 : PC_THREADS;
     *smemMax = 0;
     cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    allow_mid_clusters();
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -2237,6 +2235,15 @@ __device__ __forceinline__ T row_product(const Proj& P, const T* s, int row) {
     }
     return t;
 }
+// one row of A s per lane (row < 0: 0), all lanes of the warp together
+template <typename T, bool FUSED>
+__device__ __forceinline__ T spmv_row(const Proj& P, const T* s, int row) {
+    if (FUSED) return row_product(P, s, row);
+    T t = 0;
+    if (row >= 0)
+        for (int q = P.rowPtr[row]; q < P.rowPtr[row + 1]; ++q) t = mac_add<false>(t, (T)P.val[q], s[P.col[q]]);
+    return t;
+}
 template <typename T, bool FUSED>
 __global__ void __cluster_dims__(SPMV_CTAS, 1, 1) __launch_bounds__(SPMV_THREADS, 4)
     k_spmv_dot(Proj P, const T* s, T* y, double* part) {
@@ -2251,10 +2258,7 @@ __global__ void __cluster_dims__(SPMV_CTAS, 1, 1) __launch_bounds__(SPMV_THREADS
     const double rho = P.sc[SC_RHO];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long i = base + RED_LANES * warp + 32 * rank + lane;
-    T t = 0;
-    if (FUSED) t = row_product(P, s, i < n ? (int)i : -1);
-    else if (i < n)
-        for (int q = P.rowPtr[i]; q < P.rowPtr[i + 1]; ++q) t = mac_add<false>(t, (T)P.val[q], s[P.col[q]]);
+    const T t = spmv_row<T, FUSED>(P, s, i < n ? (int)i : -1);
     if (i < n) {
         y[i] = t;
         ss[threadIdx.x] = s[i];
@@ -2276,6 +2280,41 @@ __global__ void __cluster_dims__(SPMV_CTAS, 1, 1) __launch_bounds__(SPMV_THREADS
         if (lane == 0) part[chunk] = r;
     }
     if (FUSED) fold_alpha(P, part, rho, sh);  // the reference's order folds its own way first
+}
+// The same with one CTA per chunk, where no cluster runs.
+constexpr int SPMV_BLOCK = 1024;
+template <typename T, bool FUSED>
+__global__ void __launch_bounds__(SPMV_BLOCK) k_spmv_dot_block(Proj P, const T* s, T* y, double* part) {
+    grid_dep_wait();
+    __shared__ T ss[RED_CHUNK], ys[RED_CHUNK];
+    __shared__ double sh[RED_LANES];
+    if (*P.done) return;
+    const int n = *P.nDof, t = threadIdx.x;
+    const long long base = (long long)blockIdx.x * RED_CHUNK;
+    if (base >= n) return;
+    const double rho = P.sc[SC_RHO];
+    for (int k = t; k < RED_CHUNK; k += SPMV_BLOCK) {
+        const long long i = base + k;
+        const T v = spmv_row<T, FUSED>(P, s, i < n ? (int)i : -1);
+        if (i < n) {
+            y[i] = v;
+            ss[k] = s[i];
+            ys[k] = v;
+        }
+    }
+    __syncthreads();
+    double acc = 0.0;
+    if (t < RED_LANES)
+        for (int k = 0; k < RED_PER_LANE && base + t + RED_LANES * k < n; ++k)
+            acc = mac_add<FUSED>(acc, (double)ss[t + RED_LANES * k], (double)ys[t + RED_LANES * k]);
+    const double r = block_tree(acc, sh);
+    if (t == 0) part[blockIdx.x] = r;
+    if (FUSED) fold_alpha(P, part, rho, sh);
+}
+template <typename T, bool FUSED>
+static void launch_spmv(const Proj& P, int chunks, cudaStream_t st, const T* s, T* y) {
+    if (P.spmvCluster) launch_pdl(k_spmv_dot<T, FUSED>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, y, P.part);
+    else launch_pdl(k_spmv_dot_block<T, FUSED>, chunks, SPMV_BLOCK, st, P, s, y, P.part);
 }
 __global__ void k_alpha(Proj P, const double* part) {  // reference order only
     grid_dep_wait();
@@ -2752,15 +2791,39 @@ void launch_factor(const Dev& d, Proj& P, double omega, double minDiag, int& epo
     prof_end(prof, st);
 }
 
-static void allow_mid_clusters() {
-    const void* k[4] = {(const void*)k_mid<double, true>, (const void*)k_mid<double, false>, (const void*)k_mid<float, true>,
-                        (const void*)k_mid<float, false>};
-    for (const void* f : k) cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+// whether a cluster of `ctas` CTAs of the kernel can be resident on the current device
+static bool cluster_runs(const void* kern, int ctas, int threads) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int nc = 0;
+    const bool ok = (ctas <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                    cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) == cudaSuccess && nc > 0;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+static bool mid_runs() {
+    return cluster_runs((const void*)k_mid<double, true>, MID_CTAS, MID_THREADS) &&
+           cluster_runs((const void*)k_mid<double, false>, MID_CTAS, MID_THREADS) &&
+           cluster_runs((const void*)k_mid<float, true>, MID_CTAS, MID_THREADS) &&
+           cluster_runs((const void*)k_mid<float, false>, MID_CTAS, MID_THREADS);
+}
+static bool spmv_cluster_runs() {
+    return cluster_runs((const void*)k_spmv_dot<double, true>, SPMV_CTAS, SPMV_THREADS) &&
+           cluster_runs((const void*)k_spmv_dot<double, false>, SPMV_CTAS, SPMV_THREADS) &&
+           cluster_runs((const void*)k_spmv_dot<float, true>, SPMV_CTAS, SPMV_THREADS);
 }
 // The iteration's light work as k_mid: see there.  The level-barrier preconditioner wants the residual
 // in its own order (k_update_xr); profiling times the product by itself.
 static bool mid_fits(const Proj& P, const KProf* prof) {
-    return P.rows <= MID_MAX && P.pcAsync && P.pcCluster == MID_CTAS && !P.refOrder && !(prof && prof->on);
+    return P.rows <= MID_MAX && P.midRuns && !P.refOrder && !(prof && prof->on);
 }
 // Blocks of k_update_xr / k_update_er32: eight of TB threads per SM at most, each over several rows.  One
 // atomic on the same word per TB rows, half the blocks past the last row and FP64 comparisons made the
@@ -2807,8 +2870,8 @@ int launch_pcg_fp64(const Dev& d, Proj& P, double tolFactor, int maxIter, int& e
                 continue;
             }
             prof_begin(pf, 2, st);
-            if (P.refOrder) launch_pdl(k_spmv_dot<double, false>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, z, P.part);
-            else launch_pdl(k_spmv_dot<double, true>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, s, z, P.part);
+            if (P.refOrder) launch_spmv<double, false>(P, chunks, st, s, z);
+            else launch_spmv<double, true>(P, chunks, st, s, z);
             prof_end(pf, st);
             if (P.refOrder) {
                 launch_dot_ref(s, z, P.nDof, P.part, st);
@@ -2995,7 +3058,7 @@ int launch_pcg_mixed(const Dev& d, Proj& P, double tolFactor, int maxIter, int b
                     continue;
                 }
                 prof_begin(pf, 2, st);
-                launch_pdl(k_spmv_dot<float, true>, chunks * SPMV_CTAS, SPMV_THREADS, st, P, P.s32, P.q32, P.part);
+                launch_spmv<float, true>(P, chunks, st, P.s32, P.q32);
                 prof_end(pf, st);
                 launch_pdl(k_update_er32, rowBlocks, TB, st, P, maxIter);
                 prof_begin(pf, 0, st);
@@ -3079,6 +3142,8 @@ void proj_alloc(Proj& J, long long rows, int device, cudaStream_t st, std::vecto
     J.clusterSize = mode == "syncfree" ? 0 : choose_cluster_size(device);
     J.pcAsync = mode == "async";
     J.pcCluster = (mode == "async" || mode == "dsmem") ? choose_dsmem_cluster(J.pcAsync, &J.pcSmemMax) : 0;
+    J.midRuns = J.pcAsync && J.pcCluster > 0 && mid_runs();
+    J.spmvCluster = mode != "syncfree" && spmv_cluster_runs();
     J.pcActive = 0;
     J.pcSmem = 0;
     J.bsum = A.get<int>((rows * ROW_W + 1 + 1023) / 1024 + 1);

@@ -210,7 +210,9 @@ __device__ __forceinline__ int half_face(int dir, int k) {
 // Each thread is one long chain of dependent loads and FP64 operations (the samples near level
 // transitions above all), so small grids and the few half tilts took a chain's length per launch: side by
 // side they take it once (buoyancy 0.53 -> 0.41 ms per step at 64^3 x 3, 0.33 -> 0.23 ms at 8^3 x 3).  The
-// longest chains come first.
+// longest chains come first.  A half tilt that is marked open too (no layout or step makes one, a caller's
+// marks can) takes both shares, the open tilt's first, from its half tilt's thread: no two threads write
+// one slot.
 __global__ void k_force(Dev d, Fields F, const uint8_t* open, const double* amb, double dt) {
     const int bH = (8 * d.H + TB - 1) / TB, bT = (int)((8LL * d.S + TB - 1) / TB);
     int b = blockIdx.x;
@@ -223,18 +225,20 @@ __global__ void k_force(Dev d, Fields F, const uint8_t* open, const double* amb,
         const int hs = d.half[idx >> 3], k = idx & 7;
         const int q = half_face(tf_dir(F.tf[hs]), k);
         out = F.tv + (size_t)hs * 8 + k;
+        const V3 c = vert_pos(d, hs);
+        if (open[hs] && !ghost(d, hs))
+            *out = *out + dt * (tilt_up(k, 2) * force_at(d, F, tilt_pos(c, k, F.te[hs]), *amb));
         if (q < 0) {
             *out = *out + dt * 0.0;
             return;
         }
-        const V3 c = vert_pos(d, hs);
         p = q == 4 ? c : tilt_pos(c, k, F.te[hs]);
         dv = q == 4 ? v3(HALF_DIR_POS[k][0], HALF_DIR_POS[k][1], HALF_DIR_POS[k][2]) : tilt_up3(k);
     } else if ((b -= bH) < bT) {
         const long long idx = (long long)b * TB + threadIdx.x;
         if (idx >= 8LL * d.S) return;
         const int s = (int)(idx >> 3), k = (int)(idx & 7);
-        if (ghost(d, s) || !open[s]) return;
+        if (ghost(d, s) || !open[s] || d.halfMark[s]) return;
         p = tilt_pos(vert_pos(d, s), k, F.te[s]);
         dv.z = tilt_up(k, 2);
         out = F.tv + idx;
@@ -651,13 +655,13 @@ __global__ void k_advect(Dev d, Fields cur, Fields nxt, const uint8_t* open, dou
         kind = FACE;
         s = (int)(idx >> 3);
         k = (int)(idx & 7);
-        if (ghost(d, s) || (nxt.tf[s] & TF_CLOSED)) return;
+        if (ghost(d, s) || (nxt.tf[s] & TF_CLOSED) || d.halfMark[s]) return;  // half tilts: above
         p = tilt_pos(vert_pos(d, s), k, nxt.te[s]);
         dv = tilt_up3(k);
     } else if ((b -= bT) < bS) {
         kind = SCALAR_TILT;
         s = b * TB + threadIdx.x;
-        if (s >= d.S || ghost(d, s) || !open[s]) return;
+        if (s >= d.S || ghost(d, s) || !open[s] || d.halfMark[s]) return;
         p = vert_pos(d, s);
     } else if ((b -= bS) < bS) {
         kind = SCALAR_OCT;

@@ -18,6 +18,7 @@
 // and one fused advection kernel (layout adjustment, density, heat, tilted faces and MAC faces;
 // density and heat share each back-trace).
 #include <cstdint>
+#include <type_traits>
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -475,7 +476,7 @@ constexpr int WAVE_VAL = WAVE_CHUNK * 1024, WAVE_TL = WAVE_VAL + WAVE_CHUNK * 25
 constexpr int WAVE_STAGE = WAVE_TZ + WAVE_CHUNK * 1024;
 constexpr int WAVE_RING = WAVE_STAGES * WAVE_STAGE;
 constexpr int WAVE_PAD = 48;       // edge slots before row 0 and after row ny - 1
-constexpr int WAVE_MAX_NY = (224 * 1024 - WAVE_RING) / 8 - 2 * WAVE_PAD;
+constexpr int WAVE_MAX_NY = (224 * 1024 - WAVE_RING) / 8 - 2 * WAVE_PAD;  // rows whose edge fits shared memory
 
 // records of the factorised system for the wavefront kernel (one thread per row)
 __global__ void k2_wave_gather(Proj P, const int* vIdx) {
@@ -543,6 +544,30 @@ __device__ __forceinline__ double wave_ld1(uint32_t a) {
     asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
     return v;
 }
+// Results handed from warp to warp stand in the reader's shared memory or, for grids too tall for that
+// (TALL), in global memory; A is the type of their byte addresses, and its width says which.  The reader
+// is behind by then: a step is no slower (ms per iteration, GB300: 100 x 20,000 9.1 and, by the generic
+// sweeps, 125; 33 x 19,000 9.5 and 102; one warp's 2 x 25,400, which hands nothing on, 9.9 and 13.8).
+__device__ __forceinline__ double2 wave_ld2(unsigned long long a) {
+    double2 v;
+    asm volatile("ld.volatile.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(a) : "memory");
+    return v;
+}
+// a step's result: into wZ where the row is in the grid, into the neighbour's edge from the boundary lane
+__device__ __forceinline__ void wave_put(double* out, uint32_t peer, double v, bool on, bool writer) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n setp.ne.b32 q, %4, 0;\n"
+        " @q st.shared::cluster.f64 [%1], %2;\n @p st.global.f64 [%0], %2;\n}" ::"l"(out),
+        "r"(peer), "d"(v), "r"((int)on), "r"((int)writer)
+        : "memory");
+}
+__device__ __forceinline__ void wave_put(double* out, unsigned long long peer, double v, bool on, bool writer) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n setp.ne.b32 q, %4, 0;\n"
+        " @q st.volatile.global.f64 [%1], %2;\n @p st.global.f64 [%0], %2;\n}" ::"l"(out),
+        "l"(peer), "d"(v), "r"((int)on), "r"((int)writer)
+        : "memory");
+}
 __device__ __forceinline__ bool wave_empty(double v) { return __double2hiint(v) == (int)(WAVE_EMPTY >> 32); }
 // waits for the phase of `parity`; false past the limit (status), or, given a status, once any wait
 // has given up
@@ -596,8 +621,8 @@ __device__ __forceinline__ void wave_copy(const Proj& P, const WaveWarp& W) {
 
 // One sweep over the warp's lines, upwards (forward) or downwards (backward).  The boundary lane (0
 // forward, 31 backward) takes its neighbour's results from `edge` (by row; the slots outside the
-// grid hold 0, and so do all of them in the warp that has no such neighbour: no step checks the
-// range), the opposite lane stores its own into `peer` (0: none).  The warp issues in order and pays
+// grid hold 0: no step checks the range; a warp that is not linked to such a neighbour reads one pair of
+// zeros all the way), the opposite lane stores its own into `peer` (0: none).  The warp issues in order and pays
 // 20 to 30 cycles for each load or store among a step's FP64 operations, so these stand together:
 // once per WAVE_GROUP steps, the next group's records and edge values and this group's results.
 constexpr int WAVE_GROUP = 2;
@@ -605,16 +630,17 @@ struct WaveGroup {
     double2 l[WAVE_GROUP], iv[WAVE_GROUP];
     double v[WAVE_GROUP], edge[WAVE_GROUP];
 };
-template <bool FWD>
-__device__ __forceinline__ void wave_sweep(const Proj& P, const WaveWarp& W, uint32_t edge, uint32_t peer) {
+template <bool FWD, typename A>
+__device__ __forceinline__ void wave_sweep(const Proj& P, const WaveWarp& W, A edge, A peer, bool linked) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, sd = FWD ? 1 : -1;
     const unsigned bound = W.x < P.wnx ? P.wny : 0;
     const bool first = lane == (FWD ? 0 : 31), writer = peer != 0 && lane == (FWD ? 31 : 0);
     const int start = FWD ? 0 : W.chunks * WAVE_CHUNK - 1;  // the sweep's first line
     int y = start - lane;                                   // this lane's row
-    uint32_t ea = edge + 8 * (start - (FWD ? 0 : 31));  // the boundary lane's row
-    uint32_t pa = peer + 8 * y;
+    A ea = edge + (A)(linked ? 8 * (start - (FWD ? 0 : 31)) : 0);  // the boundary lane's row
+    const int ed = linked ? 8 * WAVE_GROUP * sd : 0;
+    A pa = peer + (A)(8 * y);
     double* out = P.wZ + (W.line0 + start) * 32LL + lane;
     double prev = 0;  // this column's last result
     constexpr int G = WAVE_GROUP;
@@ -666,7 +692,7 @@ __device__ __forceinline__ void wave_sweep(const Proj& P, const WaveWarp& W, uin
             }
             __syncwarp();
             cur = nxt;
-            ea += 8 * G * sd;
+            ea += (A)ed;
             if (h + 1 < WAVE_CHUNK / G) {
                 load(nxt, stage, h + 1);
             } else if (c + 1 < W.chunks) {
@@ -693,15 +719,9 @@ __device__ __forceinline__ void wave_sweep(const Proj& P, const WaveWarp& W, uin
                 res[k] = prev = acc * cur.iv[k].x;
             }
 #pragma unroll
-            for (int k = 0; k < G; ++k) {
-                asm volatile(
-                    "{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n setp.ne.b32 q, %4, 0;\n"
-                    " @q st.shared::cluster.f64 [%1], %2;\n @p st.global.f64 [%0], %2;\n}" ::"l"(out + sd * 32 * k),
-                    "r"(pa + 8 * sd * k), "d"(res[k]), "r"((int)((unsigned)(y + sd * k) < bound)), "r"((int)writer)
-                    : "memory");
-            }
+            for (int k = 0; k < G; ++k) wave_put(out + sd * 32 * k, pa + (A)(8 * sd * k), res[k], (unsigned)(y + sd * k) < bound, writer);
             out += sd * 32 * G;
-            pa += 8 * sd * G;
+            pa += (A)(8 * sd * G);
             y += sd * G;
         }
         __syncwarp();
@@ -711,6 +731,7 @@ __device__ __forceinline__ void wave_sweep(const Proj& P, const WaveWarp& W, uin
     }
 }
 // z: the tilt rows' results; the cells' stay in wZ
+template <bool TALL>
 __global__ void __launch_bounds__(WAVE_THREADS, 1) k2_precond_wave(Proj P, const double* r, double* z) {
     extern __shared__ __align__(16) unsigned char wave_smem[];
     __shared__ __align__(8) unsigned long long bars[2 * WAVE_STAGES];
@@ -718,7 +739,9 @@ __global__ void __launch_bounds__(WAVE_THREADS, 1) k2_precond_wave(Proj P, const
     if (*P.done) return;
     const int nx = P.wnx, ny = P.wny, nc = nx * ny, n = *P.nDof;
     const int rank = cl.block_rank(), nb = cl.num_blocks(), x0 = 32 * rank;
-    double* e = reinterpret_cast<double*>(wave_smem + WAVE_RING);
+    typedef typename std::conditional<TALL, unsigned long long, uint32_t>::type A;
+    const int rows = nb > 1 ? ny : 0, stride = (rows + 2 * WAVE_PAD + 1) & ~1;  // of an edge
+    double* e = TALL ? P.wEdge + (size_t)rank * stride : reinterpret_cast<double*>(wave_smem + WAVE_RING);
     WaveWarp W;
     W.ring = (uint32_t)__cvta_generic_to_shared(wave_smem);
     W.bars = (uint32_t)__cvta_generic_to_shared(bars);
@@ -726,15 +749,19 @@ __global__ void __launch_bounds__(WAVE_THREADS, 1) k2_precond_wave(Proj P, const
     W.line0 = rank * wave_lines(ny);
     W.chunks = (ny + min(31, nx - 1 - x0) + WAVE_CHUNK - 1) / WAVE_CHUNK;  // up to the last line with a cell
     W.g0 = 0;
-    const uint32_t edge = W.ring + WAVE_RING + 8 * WAVE_PAD;  // row 0
-    auto peer = [&](int q, uint32_t mine) {
+    A edge;  // row 0
+    if (TALL) edge = (A)(uintptr_t)(e + WAVE_PAD);
+    else edge = (A)(W.ring + WAVE_RING + 8 * WAVE_PAD);
+    auto peer = [&](int q, A mine) {
+        if (q < 0 || q >= nb) return (A)0;
+        if (TALL) return mine + (A)(8LL * (q - rank) * stride);
         uint32_t m = 0;
-        if (q >= 0 && q < nb) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(mine), "r"(q));
-        return m;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"((uint32_t)mine), "r"(q));
+        return (A)m;
     };
     auto clear = [&](bool neighbour, int row0) {  // row 0 at slot row0
-        for (int i = threadIdx.x; i < ny + 2 * WAVE_PAD; i += blockDim.x)
-            e[i] = neighbour && i >= row0 && i < ny + row0 ? __longlong_as_double((long long)WAVE_EMPTY) : 0.0;
+        for (int i = threadIdx.x; i < stride; i += blockDim.x)
+            e[i] = neighbour && i >= row0 && i < rows + row0 ? __longlong_as_double((long long)WAVE_EMPTY) : 0.0;
     };
     clear(rank > 0, WAVE_PAD);
     if (threadIdx.x == 32) {
@@ -742,13 +769,13 @@ __global__ void __launch_bounds__(WAVE_THREADS, 1) k2_precond_wave(Proj P, const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cl.sync();  // every CTA is running and its edge is empty
-    if (threadIdx.x < 32) wave_sweep<true>(P, W, edge, peer(rank + 1, edge));
+    if (threadIdx.x < 32) wave_sweep<true, A>(P, W, edge, peer(rank + 1, edge), rank > 0);
     else if (threadIdx.x == 32) wave_copy<true>(P, W);
     __syncwarp();
     __threadfence();
     cl.sync();
     clear(rank + 1 < nb, WAVE_PAD + 1);
-    // (rows one slot on: a group's four rows, read as two aligned pairs, then start at an odd row)
+    // (rows one slot on: a group's two rows, read as one aligned pair, then start at an odd row)
     // tilt rows: forward (their four cells), then their backward step (no upper entries); the result
     // also goes to the four cells' records for the backward sweep
     for (int tr = nc + rank * blockDim.x + threadIdx.x; tr < n; tr += nb * blockDim.x) {
@@ -771,7 +798,7 @@ __global__ void __launch_bounds__(WAVE_THREADS, 1) k2_precond_wave(Proj P, const
     asm volatile("fence.proxy.async;" ::: "memory");  // wZ and wTz are read by bulk copies
     cl.sync();
     W.g0 = W.chunks;
-    if (threadIdx.x < 32) wave_sweep<false>(P, W, edge + 8, peer(rank - 1, edge + 8));
+    if (threadIdx.x < 32) wave_sweep<false, A>(P, W, edge + 8, peer(rank - 1, edge + 8), rank + 1 < nb);
     else if (threadIdx.x == 32) {
         asm volatile("fence.proxy.async;" ::: "memory");
         wave_copy<false>(P, W);
@@ -831,13 +858,18 @@ void launch2_wave_gather(const Proj& P, const int* vIdx, int rows, cudaStream_t 
     cudaMemsetAsync(P.wTf, 0, sizeof(int) * (wave_slots(P.wnx, P.wny) / (32 * WAVE_CHUNK)), st);
     ASTG_LAUNCH(k2_wave_gather<<<nblk2(rows), TB2, 0, st>>>(P, vIdx));
 }
-static size_t wave_smem_bytes(int ny) { return (size_t)WAVE_RING + 8 * (size_t)(ny + 2 * WAVE_PAD); }
+static bool wave_tall(int nx, int ny) { return nx > 32 && ny > WAVE_MAX_NY; }
+long long wave_edge_slots(int nx, int ny) { return wave_tall(nx, ny) ? (nx + 31LL) / 32 * ((ny + 2 * WAVE_PAD + 1) & ~1) : 0; }
+static size_t wave_smem_bytes(int nx, int ny) {
+    if (wave_tall(nx, ny)) return WAVE_RING;
+    return (size_t)WAVE_RING + 8 * (size_t)(((nx > 32 ? ny : 0) + 2 * WAVE_PAD + 1) & ~1);
+}
 static void wave_config(int nx, int ny, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at) {
     const int ctas = (nx + 31) / 32;
     cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(WAVE_THREADS);
-    cfg.dynamicSmemBytes = wave_smem_bytes(ny);
+    cfg.dynamicSmemBytes = wave_smem_bytes(nx, ny);
     cfg.stream = st;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = ctas;
@@ -851,20 +883,21 @@ void launch_precond_wave(const Proj& P, const double* r, double* z, cudaStream_t
     cudaLaunchAttribute at[1];
     wave_config(P.wnx, P.wny, st, cfg, at);
     count_launch();
-    note_launch(cudaLaunchKernelEx(&cfg, k2_precond_wave, P, r, z));
+    note_launch(cudaLaunchKernelEx(&cfg, P.wEdge ? k2_precond_wave<true> : k2_precond_wave<false>, P, r, z));
 }
-// The wavefront kernel takes up to WAVE_MAX_NX columns (16 CTAs of 32) and as many rows as fit a
-// CTA's shared memory; its slots use 32-bit indices.  Wider and taller grids take the generic sweeps.  Call with the device current.
+// The wavefront kernel takes up to WAVE_MAX_NX columns (16 CTAs of 32) and any height; its slots use
+// 32-bit indices.  Wider grids take the generic sweeps.  Call with the device current.
 bool wave_supported(int nx, int ny) {
-    if (nx < 2 || nx > WAVE_MAX_NX || ny > WAVE_MAX_NY || wave_slots(nx, ny) * 4 >= (1LL << 31)) return false;
+    if (nx < 2 || nx > WAVE_MAX_NX || wave_slots(nx, ny) * 4 >= (1LL << 31)) return false;
+    const void* kern = wave_tall(nx, ny) ? (const void*)k2_precond_wave<true> : (const void*)k2_precond_wave<false>;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     wave_config(nx, ny, nullptr, cfg, at);
     int nc = 0;
     const bool ok =
-        cudaFuncSetAttribute(k2_precond_wave, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(k2_precond_wave, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wave_smem_bytes(WAVE_MAX_NY)) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&nc, k2_precond_wave, &cfg) == cudaSuccess && nc > 0;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wave_smem_bytes(64, WAVE_MAX_NY)) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) == cudaSuccess && nc > 0;
     if (!ok) cudaGetLastError();
     return ok;
 }

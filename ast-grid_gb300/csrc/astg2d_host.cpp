@@ -147,6 +147,7 @@ struct astg2_handle {
             J.wStatus = status;
             J.wTl = dalloc<double>(4 * skew);
             J.wTz = dalloc<double>(4 * skew);
+            if (wave_edge_slots(nx, ny)) J.wEdge = dalloc<double>(wave_edge_slots(nx, ny));
             J.wTf = dalloc<int>(skew / (32 * WAVE_CHUNK));
             J.wTc = dalloc<int>(4 * nv());
             J.wTv = dalloc<double>(4 * nv());

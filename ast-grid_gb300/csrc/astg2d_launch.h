@@ -48,6 +48,7 @@ void launch2_advect(const Grid2& g, const Fields2& cur, const Fields2& nxt, cons
 // whether the wavefront kernel takes grids nx columns wide
 void launch2_wave_gather(const Proj& P, const int* vIdx, int rows, cudaStream_t st);
 bool wave_supported(int nx, int ny);
+long long wave_edge_slots(int nx, int ny);  // of Proj::wEdge; 0: the results handed on fit shared memory
 // max over cells of mx(x, y)^2 + my(x, y)^2 (ASTSolver::cfl) as the bit pattern of a double
 void launch2_cfl(const Grid2& g, const Fields2& F, unsigned long long* out, cudaStream_t st);
 

@@ -195,6 +195,7 @@ struct Proj {
     double* wZ;
     double* wTl;
     double* wTz;
+    double* wEdge;  // tall grids: the results handed from warp to warp (wave_edge_slots)
     int* wTf;
     int* wTc;
     double* wTv;

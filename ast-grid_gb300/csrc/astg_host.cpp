@@ -950,11 +950,16 @@ struct astg_handle {
         ck(cudaMemcpyAsync(J.col, col, sizeof(int) * nnz, cudaMemcpyHostToDevice, st), "upload");
         ck(cudaMemcpyAsync(J.val, val, sizeof(double) * nnz, cudaMemcpyHostToDevice, st), "upload");
         select_preconditioner(J, n);
-        // more right-hand sides than such solves fit side by side: the form that shares SMs (20 right-hand
-        // sides, ms: 42 k rows 34 -> 28; from 100 k rows on, where a solve fills its SMs' shared memory
-        // and the L2, it is the slower one: 315 k rows FP64 230 -> 347)
-        if (J.pcAsync && n <= 100000 && nrhs > precond_concurrency(J, precision == ASTG_MIXED && J.pcActive32))
+        // More right-hand sides than such solves fit side by side: the form of which two CTAs share an SM.
+        // ms for 8 / 20 right-hand sides (GB300), single and batch form: 42 k rows FP64 22 / 34 and 14 / 28,
+        // mixed 20 / 33 and 13 / 28; 305 k rows mixed 100 / 184 and 78 / 172, FP64 100 / 167 and 133 / 227:
+        // there two vectors fill an SM's shared memory and the L2, and the single form stays.
+        const bool fp32 = precision == ASTG_MIXED && J.pcActive32;
+        const int alone = precond_concurrency(J, fp32);
+        if (J.pcAsync && nrhs > alone && (fp32 || n <= 100000)) {
             select_preconditioner(J, n, true);
+            if (precond_concurrency(J, fp32) <= alone) select_preconditioner(J, n);
+        }
         launch_external_system(d, J, n, st);
         checkStatus();
         const bool mixed = precision == ASTG_MIXED && J.pcActive32;

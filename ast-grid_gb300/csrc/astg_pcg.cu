@@ -2582,7 +2582,7 @@ void select_preconditioner(Proj& P, int n, bool batch) {
     // CTAs to an SM, which 8 warps' registers allow (20 right-hand sides at 42 k rows 34 -> 28 ms).
     P.pcWarps = batch ? 8 : n > 200000 ? 16 : n > 30000 ? 12 : 8;
     P.pcCS = n > 4096 ? P.pcCluster : 1;
-    const int blocks = n > 100000 && !batch ? 2 : 1;
+    const int blocks = n > 100000 ? 2 : 1;
     P.pcBlock = (n + P.pcCS * blocks - 1) / (P.pcCS * blocks);
     P.pcChunk = P.pcBlock * blocks;
     const size_t slots = (size_t)P.pcChunk + 1;  // and the slot that holds 0

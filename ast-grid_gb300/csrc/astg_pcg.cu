@@ -2575,13 +2575,14 @@ void select_preconditioner(Proj& P, int n, bool batch) {
         P.pcSmem = bytes;
         return;
     }
-    // us per PCG iteration on GB300, FP64 / FP32 form.  Warps per CTA: 22 k rows 8: 87 / 70, 12: 89 / 69;
-    // 42 k rows 8: 110 / 90, 12: 109 / 83; 305 k rows 12: 290 / 238, 16: 284 / 227.  Row blocks per CTA:
-    // 78 k rows 1: 142 / 114, 2: 146 / 112; 132 k rows 2: 181 / 141, 3: 193 / 156.  CTAs: 1.5 k rows
-    // one 46, eight 48 (FP64); 10.6 k rows 16 and 8 alike.  Many solves at once gain more from two
-    // CTAs to an SM, which 8 warps' registers allow (20 right-hand sides at 42 k rows 34 -> 28 ms).
+    // us per PCG iteration on GB300, FP64 / FP32 form, on both sides of each line.  Warps per CTA: 18.8 k
+    // rows 8: 80 / 63, 12: 82 / 63; 29.2 k 8: 97 / 78, 12: 97 / 74; 42.2 k 8: 112 / 91, 12: 109 / 83; 132 k
+    // 12: 176 / 138, 16: 187 / 141; 206 k 12: 226 / 188, 16: 227 / 176; 305 k 12: 316 / 257, 16: 286 / 228.
+    // Row blocks per CTA: 78 k rows 1: 142 / 114, 2: 146 / 112; 132 k rows 2: 181 / 141, 3: 193 / 156.
+    // CTAs: 1.2 k rows one 37 / 34, sixteen 42 / 37; 2.1 k 44 / 41 and 45 / 40; 4.1 k 56 / 51 and 52 / 44.
+    // Many solves at once gain more from two CTAs to an SM, which 8 warps' registers allow.
     P.pcWarps = batch ? 8 : n > 200000 ? 16 : n > 30000 ? 12 : 8;
-    P.pcCS = n > 4096 ? P.pcCluster : 1;
+    P.pcCS = n > 2100 ? P.pcCluster : 1;
     const int blocks = n > 100000 ? 2 : 1;
     P.pcBlock = (n + P.pcCS * blocks - 1) / (P.pcCS * blocks);
     P.pcChunk = P.pcBlock * blocks;

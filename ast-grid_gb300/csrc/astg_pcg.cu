@@ -117,8 +117,8 @@ static void prof_drain(KProf* p, bool replayed = false) {
 
 // One batch of PCG iterations, either launched directly or replayed from a CUDA graph captured
 // on the first full batch (the kernels skip themselves once the device's done flag is set, so a
-// batch is the same work every time).  Replaying saves the launch gaps of the ~9 small kernels of
-// an iteration.  Not used with the sync-free sweeps, whose epoch counter changes every launch.
+// batch is the same work every time).  Replaying saves the launch gaps of an iteration's five
+// kernels (two with k_mid).  Not used with the sync-free sweeps, whose epoch counter changes every launch.
 // While kernel profiling is on, one replay in KPROF_GRAPH_EVERY runs a second graph whose kernels
 // are bracketed by event-record nodes (those nodes cost about 3 us each), the others the plain one.
 bool g_pcg_graphs = getenv("ASTG_PCG_GRAPH") ? atoi(getenv("ASTG_PCG_GRAPH")) != 0 : true;
@@ -1308,8 +1308,8 @@ __global__ void __launch_bounds__(256, 1) k_precond_dsmem(Proj P, double* z, int
 // * The records bypass L1: at 150 KB of shared memory per CTA little L1 is left, and allocating
 //   there cost 7 % (238 -> 222 us).
 // * A scattered read of another CTA's slots takes ~3 cycles per lane, and 225 cycles at least, so
-//   rows are dealt in large blocks (select_preconditioner): with three per CTA 14 % of the entries cross CTAs instead of
-//   34 % with blocks of 256 rows.
+//   rows are dealt in large blocks (select_preconditioner): with two per CTA 14 % of the entries of the
+//   256^3-equivalent system cross CTAs, with one 8 %, with blocks of 256 rows 33 %.
 constexpr long long PCA_SPIN_LIMIT = 1LL << 22;
 constexpr int PCA_MAX_WARPS = 16;
 // Value-type traits of the barrier-free preconditioner (FP64 drop-in form, FP32 inner solve of the

@@ -952,13 +952,17 @@ struct astg_handle {
         select_preconditioner(J, n);
         // More right-hand sides than such solves fit side by side: the form of which two CTAs share an SM.
         // ms for 8 / 20 right-hand sides (GB300), single and batch form: 42 k rows FP64 22 / 34 and 14 / 28,
-        // mixed 20 / 33 and 13 / 28; 305 k rows mixed 100 / 184 and 78 / 172, FP64 100 / 167 and 133 / 227:
-        // there two vectors fill an SM's shared memory and the L2, and the single form stays.
+        // mixed 20 / 33 and 13 / 28.  Above 100 k rows FP64 keeps the single form (305 k rows 100 / 167 and
+        // 133 / 227: two vectors fill an SM's shared memory, and the L2), and mixed takes the batch form
+        // where it saves rounds enough: one of 7 solves takes 67 ms at 311 k rows, one of 8 to 14 in batch
+        // form 89 to 125 (8 right-hand sides 108 and 89, 14 145 and 125, 20 206 and 212).
         const bool fp32 = precision == ASTG_MIXED && J.pcActive32;
         const int alone = precond_concurrency(J, fp32);
         if (J.pcAsync && nrhs > alone && (fp32 || n <= 100000)) {
             select_preconditioner(J, n, true);
-            if (precond_concurrency(J, fp32) <= alone) select_preconditioner(J, n);
+            const int shared = precond_concurrency(J, fp32);
+            auto rounds = [&](int k) { return (nrhs + k - 1) / k; };
+            if (shared <= alone || (n > 100000 && 3 * rounds(shared) >= 2 * rounds(alone))) select_preconditioner(J, n);
         }
         launch_external_system(d, J, n, st);
         checkStatus();

@@ -1,5 +1,5 @@
 """Batches of systems above 100,000 rows: the mixed form takes the launch shape that shares SMs (two row
-blocks per CTA), FP64 keeps the single solve's; every solution is the one astg_solve returns, bit for
+blocks per CTA) where that saves rounds, FP64 keeps the single solve's; every solution is the one astg_solve returns, bit for
 bit, so the tolerance is zero."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ from fixtures import csr
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,nrhs,precision", [(100000, 9, "mixed"), (100001, 9, "mixed"), (100001, 9, "fp64"), (250000, 10, "mixed"), (500000, 9, "mixed")])
+@pytest.mark.parametrize("n,nrhs,precision", [(100000, 9, "mixed"), (100001, 9, "mixed"), (100001, 9, "fp64"), (250000, 10, "mixed"), (250000, 18, "mixed"), (500000, 9, "mixed")])
 def test_batches_equal_single_solves(n, nrhs, precision):
     import ast_solver
 

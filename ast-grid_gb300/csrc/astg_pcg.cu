@@ -1296,8 +1296,8 @@ __global__ void __launch_bounds__(256, 1) k_precond_dsmem(Proj P, double* z, int
 // What bounds it: latency per level, from the store of a value to the store of a value that
 // depends on it.  Measured on GB300 for the 256^3-equivalent system (306,797 rows, 187 levels) per
 // application against the earlier form (one generic row per lane, up to 16 polled entries,
-// 256 threads): FP64 464 -> 222 us, FP32 330 -> 170 us; 42,797 rows (92 levels) FP64 82 us; 1,542
-// rows (28 levels) FP64 27 us.  What the measurements showed:
+// 256 threads): FP64 464 -> 219 us, FP32 330 -> 179 us; 42 k rows (92 levels) FP64 78 us; 1,433
+// rows (28 levels) FP64 26 us.  What the measurements showed:
 // * The instructions of a row's path count, not its bytes: a lone warp issues a dependent
 //   instruction every ~5 cycles, so the earlier polling pass of ~400 instructions cost more than
 //   the chain it waited for.
@@ -1521,8 +1521,8 @@ k_precond_async(const __grid_constant__ PcaData<T> D, const T* r, T* z, const in
         if (wid < items) {
             const int last = first + items - 1;
             // descriptions of this item and the next two: the next one's is needed for its fetches as soon as
-            // this item begins, so it is asked for an item earlier (one ahead: 264 instead of 250 us at 306 k
-            // rows, with the profiling events)
+            // this item begins, so it is asked for an item earlier (one ahead: FP64 264 instead of 248 us at
+            // 306 k rows, with the profiling events)
             int4 d = __ldg(S.desc + first + wid), dn = __ldg(S.desc + min(first + wid + W, last)),
                  dm = __ldg(S.desc + min(first + wid + 2 * W, last));
             size_t at = (size_t)d.x + min(lane, d.y - 1);
